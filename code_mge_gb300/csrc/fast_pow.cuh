@@ -36,7 +36,8 @@ __device__ __forceinline__ double pow_7_5(double x, double d) {
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const double z2 = z * z;
-    z = (4.0 * z + a / (z2 * z2)) / 5.0;
+    const double t = 4.0 * z + a / (z2 * z2), u = t * 0.2;
+    z = fma(fma(-u, 5.0, t), 0.2, u);  // t / 5, Markstein's quotient with 0.2 = RN(1/5): the same bits
   }
   const double y = x * z;
   return y + y * (d * (double)logf((float)x));

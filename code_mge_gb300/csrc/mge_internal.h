@@ -85,6 +85,7 @@ struct StageArgs {
   int vt;
   int tmode;        // unsteady source term: 0 none, 1 first step (itime 1), 2 BDF2 (itime > 1)
   int fast;         // the contracted FP64 residual of the mixed form's finest level (JST central, Euler)
+  int faces_only;   // the stages before the last leave the edge and corner ghosts (nothing reads them there)
 };
 
 struct PhysParams {
@@ -162,10 +163,9 @@ enum MultiKind {
   MK_IRS0,       // 5 * lines along i, j, k
   MK_IRS1,
   MK_IRS2,
-  MK_BC,         // boundary-pass items
-  MK_CORNER0,    // corner phases
-  MK_CORNER1,
-  MK_CORNER2,
+  MK_BC0,        // face ghosts
+  MK_BC1,        // edge and corner ghosts
+  MK_BC2,        // corner cells of the blocks with a face without a boundary condition
   MK_RTP,        // 256 * residual partial sums
   MK_ONE,        // one thread block
   MK_COUNT
@@ -231,7 +231,11 @@ template <typename T> void launch_irs_part(int part, const DevBlock<T>& b, const
 template <typename T> void launch_solut(const DevBlock<T>& b, const PhysParams& P, double rm, double p_tot, int ns,
                                         double* out, cudaStream_t s);
 template <typename T> void launch_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s);
-template <typename T> void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
+// faces_only: without the edge and corner ghosts (StageArgs::faces_only)
+template <typename T> void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s,
+                                        bool faces_only = false);
+// work items of the boundary launches (part 0, 1, 2; 0 items: no launch)
+template <typename T> long long bc_items(const DevBlock<T>& b, int part);
 template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* partial,
                                         int npartial, double* out, cudaStream_t s, unsigned* err = nullptr);
 template <typename T> void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);

@@ -995,7 +995,8 @@ __device__ void rec_wall_terms(const DevBlock<T>& b, const PhysParams& P, int di
 }
 
 template <typename T>
-__global__ void k_rec_wall(DevBlock<T> b, PhysParams P, int dissip_on, T cd, unsigned* err) {
+__global__ void k_rec_wall(const __grid_constant__ DevBlock<T> b, const __grid_constant__ PhysParams P, int dissip_on,
+                           T cd, unsigned* err) {
   int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < b.nmir) rec_wall_terms(b, P, dissip_on, cd, err, m);
 }
@@ -1848,8 +1849,6 @@ __device__ void body_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned
 }
 
 // --------------------------------------------------------------- face boundary conditions
-// One launch per face in the order 1..6 of bcond.f90:16-39: later faces read
-// and overwrite ghost cells that earlier faces wrote.
 // the far field's powers: the short forms for gamma = 1.4 in FP64 (fast_pow.cuh)
 __device__ __forceinline__ double pow_gm(const PhysParams& P, double x, double gm) {
   if (P.gamma14) return pow_5_2(x, P.pow_dm);
@@ -1862,267 +1861,401 @@ __device__ __forceinline__ double pow_gamma(const PhysParams& P, double x, doubl
 }
 __device__ __forceinline__ float pow_gamma(const PhysParams&, float x, float gamma) { return pow(x, gamma); }
 
+// depvars with plain products: the same bits as depvars(), and the shorter
+// dependent chain (32 cycles a product against about 100 for smul) where few
+// cells are worked on and the FP64 pipe is idle
+template <typename T> __device__ __forceinline__ T depvars_plain(T gamma, const T* w) {
+  const T qq = T(0.5) * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) / w[0];
+  return (gamma - T(1)) * fdimT(w[4], qq);
+}
+
+template <typename T> struct CellState {
+  T w[5];
+  T p;
+};
 template <typename T>
-__device__ void body_bc_face(const DevBlock<T>& b, const PhysParams& P, int face, long long t) {
+__device__ __forceinline__ CellState<T> load_cell(const DevBlock<T>& b, long long c) {
+  CellState<T> s;
+#pragma unroll
+  for (int v = 0; v < 5; v++) s.w[v] = b.w[v * b.N + c];
+  s.p = b.p[c];
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ void store_cell(const DevBlock<T>& b, long long c, const CellState<T>& s) {
+#pragma unroll
+  for (int v = 0; v < 5; v++) b.w[v * b.N + c] = s.w[v];
+  b.p[c] = s.p;
+}
+
+// bc_far.f90:42-284: the ghost state of a far-field face from the state s of
+// the cell it is taken from, in place; false (s unchanged) when the normal
+// velocity is NaN.  Inflow and outflow differ only in the entropy and in the
+// tangential velocities, so both run the same chain; the quotients by the
+// cell's density share one reciprocal, those by gamma-1 and gamma take the
+// host's (mdiv: the same roundings as the divisions).
+template <typename T>
+__device__ __forceinline__ bool far_state(const DevBlock<T>& b, const PhysParams& P, int face, CellState<T>& s) {
   const int ax = (face - 1) % 3;
-  const int na = (ax == 0 ? b.jb : b.ib) + 1;  // first tangential extent
-  int t1 = (int)(t % na), t2 = (int)(t / na);
-  const int kind = b.bctype[face - 1];
-  const int lcur = ax == 0 ? b.il : (ax == 1 ? b.jl : b.kl);
-  auto at = [&](int q) -> long long {
-    if (ax == 0) return cidx(b.Pi, b.Pj, q, t1, t2);
-    if (ax == 1) return cidx(b.Pi, b.Pj, t1, q, t2);
-    return cidx(b.Pi, b.Pj, t1, t2, q);
-  };
-  const long long N = b.N;
-  int phy1, phy2, dum1, dum2;
-  if (kind == -60) {
-    if (face <= 3) {
-      dum1 = 1; dum2 = 0; phy1 = lcur; phy2 = lcur - 1;
-    } else {
-      phy1 = 2; phy2 = 3; dum1 = lcur + 1; dum2 = lcur + 2;
-    }
-  } else {
-    if (face <= 3) {
-      phy1 = 2; phy2 = 3; dum1 = 1; dum2 = 0;
-    } else {
-      phy1 = lcur; phy2 = lcur - 1; dum1 = lcur + 1; dum2 = lcur + 2;
-    }
-  }
-  const long long d1 = at(dum1), d2 = at(dum2), p1 = at(phy1), p2 = at(phy2);
-  if (kind == -20) {  // bc_far.f90:42-284
-    const T gamma = (T)P.gamma, gm = (T)P.gm;
-    const T fn0 = (T)b.fnv[face - 1][0], fn1 = (T)b.fnv[face - 1][1], fn2 = (T)b.fnv[face - 1][2];
-    const T fnn = (T)b.fnv[face - 1][ax];
-    T wp[5];
-    for (int v = 0; v < 5; v++) wp[v] = b.w[v * N + p1];
-    T pph = b.p[p1];
-    // the quotients by the cell's density share one reciprocal, those by
-    // gamma-1 and gamma take the host's (mdiv: the same roundings as the
-    // divisions, with a shorter dependent chain)
-    const T y0 = T(1) / wp[0], gm1 = gamma - T(1), rg1 = rcp_gm1(P, T(0)), rgam = rcp_gamma(P, T(0));
-    T vel_norm = mdiv(wp[1] * fn0 + wp[2] * fn1 + wp[3] * fn2, wp[0], y0);
-    T out[5], pout;
-    bool set = false;
-    const T u0a = (T)P.u0[ax];
-    const T rmi = u0a * fnn - mdiv(T(2) * (T)P.c0, gm1, rg1);
-    if (vel_norm <= T(0)) {
-      T rhoe = wp[0];
-      T ue = mdiv(wp[1 + ax], rhoe, y0);
-      T pe = pph;
-      T ce = sqrt(mdiv(gamma * pe, rhoe, y0));
-      T rpo = ue * fnn + mdiv(T(2) * ce, gm1, rg1);
-      T vv[3] = {(T)P.u0[0], (T)P.u0[1], (T)P.u0[2]};
-      vv[ax] = T(0.5) * (rpo + rmi) * fnn;
-      T ci = T(0.25) * (gamma - T(1)) * (rpo - rmi);
-      T si = (T)P.si_far;
-      T cc = mdiv(ci * ci, gamma, rgam);
-      T rhoi = pow_gm(P, si * cc, gm);
-      T prei = rhoi * cc;
-      out[0] = rhoi;
-      out[1] = rhoi * vv[0];
-      out[2] = rhoi * vv[1];
-      out[3] = rhoi * vv[2];
-      out[4] = prei * gm + T(0.5) * rhoi * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]);
-      pout = prei;
-      set = true;
-    } else if (vel_norm > T(0)) {
-      T rhoi = wp[0];
-      T vv[3] = {mdiv(wp[1], rhoi, y0), mdiv(wp[2], rhoi, y0), mdiv(wp[3], rhoi, y0)};
-      T prei = pph;
-      T si = pow_gamma(P, rhoi, gamma) / prei;
-      T ci = sqrt(mdiv(gamma * prei, rhoi, y0));
-      T rpo = vv[ax] * fnn + mdiv(T(2) * ci, gm1, rg1);
-      T ve[3] = {vv[0], vv[1], vv[2]};
-      ve[ax] = T(0.5) * (rpo + rmi) * fnn;
-      T ce = T(0.25) * (gamma - T(1)) * (rpo - rmi);
-      T cc = mdiv(ce * ce, gamma, rgam);
-      T rhoe = pow_gm(P, si * cc, gm);
-      T pe = rhoe * cc;
-      out[0] = rhoe;
-      out[1] = rhoe * ve[0];
-      out[2] = rhoe * ve[1];
-      out[3] = rhoe * ve[2];
-      out[4] = pe * gm + T(0.5) * rhoe * (ve[0] * ve[0] + ve[1] * ve[1] + ve[2] * ve[2]);
-      pout = pe;
-      set = true;
-    }
-    if (set) {  // both ghost layers take the new state
-      for (int v = 0; v < 5; v++) {
-        b.w[v * N + d1] = out[v];
-        b.w[v * N + d2] = out[v];
-      }
-      b.p[d1] = pout;
-      b.p[d2] = pout;
-    } else {  // vel_norm NaN: the second layer copies the first as it stands
-      for (int v = 0; v < 5; v++) b.w[v * N + d2] = b.w[v * N + d1];
-      b.p[d2] = b.p[d1];
-    }
-  } else if (kind == -50) {  // bc_symm.f90
-    for (int v = 0; v < 5; v++) b.w[v * N + d1] = b.w[v * N + p1];
-    b.w[(1 + ax) * N + d1] = -b.w[(1 + ax) * N + p1];
-    b.p[d1] = b.p[p1];
-    for (int v = 0; v < 5; v++) b.w[v * N + d2] = b.w[v * N + p2];
-    b.w[(1 + ax) * N + d2] = -b.w[(1 + ax) * N + p2];
-    b.p[d2] = b.p[p2];
-  } else if (kind == -80) {  // bc_wall.f90
-    b.w[d1] = b.w[p1];
-    b.w[4 * N + d1] = b.w[4 * N + p1];
-    for (int v = 1; v < 4; v++) b.w[v * N + d1] = -b.w[v * N + p1];
-    b.w[d2] = b.w[p2];
-    b.w[4 * N + d2] = b.w[4 * N + p2];
-    for (int v = 1; v < 4; v++) b.w[v * N + d2] = -b.w[v * N + p2];
-    b.p[d1] = b.p[p1];
-    b.p[d2] = b.p[p1];
-  } else if (kind == -60) {  // bc_periodic.f90
-    for (int v = 0; v < 5; v++) b.w[v * N + d2] = b.w[v * N + p2];
-    for (int v = 0; v < 5; v++) b.w[v * N + d1] = b.w[v * N + p1];
-    b.p[d2] = b.p[p2];
-    b.p[d1] = b.p[p1];
-  }
+  const T gamma = (T)P.gamma, gm = (T)P.gm;
+  const T fn0 = (T)b.fnv[face - 1][0], fn1 = (T)b.fnv[face - 1][1], fn2 = (T)b.fnv[face - 1][2];
+  const T fnn = ax == 0 ? fn0 : (ax == 1 ? fn1 : fn2);
+  const T y0 = T(1) / s.w[0], gm1 = gamma - T(1), rg1 = rcp_gm1(P, T(0)), rgam = rcp_gamma(P, T(0));
+  const T vel_norm = mdiv(s.w[1] * fn0 + s.w[2] * fn1 + s.w[3] * fn2, s.w[0], y0);
+  if (vel_norm != vel_norm) return false;
+  const bool in = vel_norm <= T(0);
+  const T rmi = (T)P.u0[ax] * fnn - mdiv(T(2) * (T)P.c0, gm1, rg1);
+  T vv[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) vv[a] = mdiv(s.w[1 + a], s.w[0], y0);
+  const T un = ax == 0 ? vv[0] : (ax == 1 ? vv[1] : vv[2]);
+  const T ce = sqrt(mdiv(gamma * s.p, s.w[0], y0));
+  const T rpo = un * fnn + mdiv(T(2) * ce, gm1, rg1);
+  const T vn = T(0.5) * (rpo + rmi) * fnn;
+  const T ci = T(0.25) * (gamma - T(1)) * (rpo - rmi);
+  const T cc = mdiv(ci * ci, gamma, rgam);
+  const T si = in ? (T)P.si_far : pow_gamma(P, s.w[0], gamma) / s.p;
+  const T rho = pow_gm(P, si * cc, gm);
+  const T pr = rho * cc;
+#pragma unroll
+  for (int a = 0; a < 3; a++) vv[a] = a == ax ? vn : (in ? (T)P.u0[a] : vv[a]);
+  s.w[0] = rho;
+  s.w[1] = rho * vv[0];
+  s.w[2] = rho * vv[1];
+  s.w[3] = rho * vv[2];
+  s.w[4] = pr * gm + T(0.5) * rho * (vv[0] * vv[0] + vv[1] * vv[1] + vv[2] * vv[2]);
+  s.p = pr;
+  return true;
+}
+// the coordinate along a face's axis that its ghost coordinate q takes its
+// state from; inner: the source of the inner layer, whatever q's layer
+__device__ __forceinline__ int bc_source(int kind, bool low, int l, int q, bool inner) {
+  const int lay = inner ? 0 : (low ? 1 - q : q - (l + 1));  // 0: next to the physical cells
+  if (kind == -60) return low ? l - lay : 2 + lay;
+  const int off = kind == -20 ? 0 : lay;  // both far-field layers take the first cell's state
+  return low ? 2 + off : l - off;
 }
 
 // bcond.f90:16-42 applies the faces 1..6 one after the other over their
 // whole tangential range, so a later face overwrites the edge and corner
-// ghosts of an earlier one and reads what the earlier one wrote.  The same
-// result comes from three passes over all faces at once, by the number of
-// ghost coordinates among a ghost cell's two tangential ones (0: face
-// ghosts, 1: edges, 2: corners), each cell written only by its last writer,
-// the highest-numbered face (with a boundary condition) whose axis is a
-// ghost axis of the cell.  That writer reads cells with one ghost axis fewer,
-// whose own writers all come before it, so every read sees the value the
-// sequential order leaves there.
+// ghosts of an earlier one and reads what the earlier one wrote.  A ghost
+// cell's final state is therefore that of its last writer, the
+// highest-numbered face (with a boundary condition) whose axis is a ghost
+// axis of the cell, applied to a cell with one ghost axis fewer.  The first
+// launch forms the cells with one ghost axis; ghost_state follows the writers
+// of an edge or corner cell down to such a cell (at most two of them) and
+// applies them on the way back.
 template <typename T>
-__device__ __forceinline__ long long bc_pass_items(const DevBlock<T>& b) {
-  const long long s0 = (long long)(b.jb + 1) * (b.kb + 1), s1 = (long long)(b.ib + 1) * (b.kb + 1),
-                  s2 = (long long)(b.ib + 1) * (b.jb + 1);
-  return 2 * (s0 + s1 + s2);
+__device__ __forceinline__ int ghost_writer(const DevBlock<T>& b, int i, int j, int k) {
+  if (((i < 2) | (i > b.il)) + ((j < 2) | (j > b.jl)) + ((k < 2) | (k > b.kl)) < 2) return 0;
+  if (k > b.kl && b.bctype[5] != 0) return 6;
+  if (j > b.jl && b.bctype[4] != 0) return 5;
+  if (i > b.il && b.bctype[3] != 0) return 4;
+  if (k < 2 && b.bctype[2] != 0) return 3;
+  if (j < 2 && b.bctype[1] != 0) return 2;
+  if (i < 2 && b.bctype[0] != 0) return 1;
+  return 0;
+}
+// moves (i, j, k) to the cell face f takes its state from; true when the
+// pressure comes from another one (bc_wall.f90 gives both layers the pressure
+// of the first physical cell), whose coordinate along the axis is then srp
+template <typename T>
+__device__ __forceinline__ bool ghost_source(const DevBlock<T>& b, int f, int& i, int& j, int& k, int& srp) {
+  const int ax = (f - 1) % 3, kind = b.bctype[f - 1];
+  const int l = ax == 0 ? b.il : (ax == 1 ? b.jl : b.kl), g = ax == 0 ? i : (ax == 1 ? j : k);
+  const int src = bc_source(kind, f <= 3, l, g, false);
+  if (ax == 0) i = src;
+  else if (ax == 1) j = src;
+  else k = src;
+  srp = bc_source(kind, f <= 3, l, g, true);
+  return kind == -80 && srp != src;
+}
+template <typename T>
+__device__ __forceinline__ void ghost_apply(const DevBlock<T>& b, const PhysParams& P, int f, CellState<T>& s) {
+  const int ax = (f - 1) % 3, kind = b.bctype[f - 1];
+  if (kind == -20) {
+    // a NaN normal velocity passes the state on: it has already stopped the run
+    far_state(b, P, f, s);
+  } else if (kind != -60) {
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      if (kind == -80 || a == ax) s.w[1 + a] = -s.w[1 + a];
+  }
+}
+// with walls among the faces: the pressure may follow another chain of cells
+template <typename T, int DEPTH>
+__device__ __noinline__ void ghost_state_wall(const DevBlock<T>& b, const PhysParams& P, int i, int j, int k,
+                                              CellState<T>& s) {
+  const int f = DEPTH > 0 ? ghost_writer(b, i, j, k) : 0;
+  if (!f) {
+    s = load_cell(b, cidx(b.Pi, b.Pj, i, j, k));
+    return;
+  }
+  if constexpr (DEPTH > 0) {
+    int srp;
+    const bool other = ghost_source(b, f, i, j, k, srp);
+    ghost_state_wall<T, DEPTH - 1>(b, P, i, j, k, s);
+    ghost_apply(b, P, f, s);
+    if (other) {
+      const int ax = (f - 1) % 3;
+      CellState<T> q;
+      ghost_state_wall<T, DEPTH - 1>(b, P, ax == 0 ? srp : i, ax == 1 ? srp : j, ax == 2 ? srp : k, q);
+      s.p = q.p;
+    }
+  }
+}
+// the state an edge or corner ghost takes from the faces; false when no face
+// writes the cell (s is then what is stored there)
+template <typename T>
+__device__ __forceinline__ bool ghost_state(const DevBlock<T>& b, const PhysParams& P, int i, int j, int k,
+                                            CellState<T>& s) {
+  const int f0 = ghost_writer(b, i, j, k);
+  bool wall = false;
+#pragma unroll
+  for (int q = 0; q < 6; q++) wall |= b.bctype[q] == -80;
+  if (wall) {  // the same for every lane
+    ghost_state_wall<T, 2>(b, P, i, j, k, s);
+    return f0 != 0;
+  }
+  int srp, f1 = 0;
+  if (f0) {
+    ghost_source(b, f0, i, j, k, srp);
+    f1 = ghost_writer(b, i, j, k);
+    if (f1) ghost_source(b, f1, i, j, k, srp);
+  }
+  s = load_cell(b, cidx(b.Pi, b.Pj, i, j, k));
+  // one copy of the far field's chain, its lanes together: calls from the
+  // levels of a recursion ran them apart and cost three times as much
+#pragma unroll 1
+  for (int q = 0; q < 2; q++) {
+    const int f = q == 0 ? f1 : f0;
+    if (f) ghost_apply(b, P, f, s);
+  }
+  return f0 != 0;
 }
 
+// Every face carries a boundary condition: all ghosts follow from physical
+// cells, and the edge and corner ghosts, the corner cells of bc_corner.f90
+// included, take one launch after the face ghosts'.  Otherwise some ghosts
+// keep what another routine put there (bc_embed, bc_overlap), and the corner
+// cells, which overwrite such ghosts, run as a launch of their own.
 template <typename T>
-__device__ __forceinline__ void body_bc_pass(const DevBlock<T>& b, const PhysParams& P, int pass, long long t) {
-  const long long sz[3] = {(long long)(b.jb + 1) * (b.kb + 1), (long long)(b.ib + 1) * (b.kb + 1),
-                           (long long)(b.ib + 1) * (b.jb + 1)};
+__host__ __device__ __forceinline__ bool bc_whole(const DevBlock<T>& b) {
+  return b.bctype[0] && b.bctype[1] && b.bctype[2] && b.bctype[3] && b.bctype[4] && b.bctype[5];
+}
+__host__ __device__ __forceinline__ int pad32(int n) { return (n + 31) & ~31; }
+// work items, in whole warps: the face ghosts (an item writes both layers);
+// the ghost cells with two or three ghost axes (without the corner cells when
+// those share the launch); the corner cells, four lanes each
+template <typename T>
+__host__ __device__ __forceinline__ int bc_n1(const DevBlock<T>& b) {
+  return pad32(2 * (b.ny * b.nz + b.nx * b.nz + b.nx * b.ny));
+}
+template <typename T>
+__host__ __device__ __forceinline__ int bc_n2(const DevBlock<T>& b) {
+  return pad32(bc_whole(b) ? 12 * (b.nx + b.ny + b.nz) + 48 : 16 * (b.nx + b.ny + b.nz) + 64);
+}
+template <typename T>
+__host__ __device__ __forceinline__ int bc_n3(const DevBlock<T>& b) {
+  return pad32(4 * (4 * b.nz + 4 * b.ny + 4 * (b.nx + 2) + 8));
+}
+template <typename T> long long bc_items_t(const DevBlock<T>& b, int part) {
+  if (part == 0) return bc_n1(b);
+  if (part == 1) return (long long)bc_n2(b) + (bc_whole(b) ? bc_n3(b) : 0);
+  return bc_whole(b) ? 0 : bc_n3(b);
+}
+
+// the face ghosts whose two tangential coordinates are physical
+template <typename T>
+__device__ __forceinline__ void body_bc_face(const DevBlock<T>& b, const PhysParams& P, int t) {
+  const int sz[3] = {b.ny * b.nz, b.nx * b.nz, b.nx * b.ny};
   int face = 1;
-  while (face < 6 && t >= sz[(face - 1) % 3]) {
-    t -= sz[(face - 1) % 3];
-    face++;
-  }
-  if (b.bctype[face - 1] == 0) return;
-  const int ax = (face - 1) % 3;
-  const int na = (ax == 0 ? b.jb : b.ib) + 1;
-  const int t1 = (int)(t % na), t2 = (int)(t / na);
-  const int ta = ax == 0 ? 1 : 0, tb = ax == 2 ? 1 : 2;  // tangential axes of t1, t2
-  const int lim[3] = {b.il, b.jl, b.kl};
-  int deg = 0;
-  bool last = true;
-  auto tangential = [&](int a, int q) {
-    const int g = q <= 1 ? a + 1 : (q > lim[a] ? a + 4 : 0);  // the face whose ghosts hold q
-    if (g) {
-      deg++;
-      if (g > face && b.bctype[g - 1] != 0) last = false;
+#pragma unroll
+  for (int q = 0; q < 5; q++)
+    if (face == q + 1 && t >= sz[q % 3]) {
+      t -= sz[q % 3];
+      face = q + 2;
     }
+  const int ax = (face - 1) % 3, kind = b.bctype[face - 1];
+  if (kind == 0 || t >= sz[ax]) return;
+  const int na = ax == 0 ? b.ny : b.nx;
+  const int t1 = 2 + t % na, t2 = 2 + t / na;
+  const int l = ax == 0 ? b.il : (ax == 1 ? b.jl : b.kl);
+  auto at = [&](int q) -> long long {
+    return ax == 0 ? cidx(b.Pi, b.Pj, q, t1, t2) : (ax == 1 ? cidx(b.Pi, b.Pj, t1, q, t2) : cidx(b.Pi, b.Pj, t1, t2, q));
   };
-  tangential(ta, t1);
-  tangential(tb, t2);
-  if (deg == pass && last) body_bc_face(b, P, face, t);
+  const bool low = face <= 3;
+  const int g1 = low ? 1 : l + 1, g2 = low ? 0 : l + 2;
+  const long long d1 = at(g1), d2 = at(g2);
+  CellState<T> s1 = load_cell(b, at(bc_source(kind, low, l, g1, false))), s2;
+  if (kind == -20) {
+    if (far_state(b, P, face, s1))
+      s2 = s1;
+    else
+      s1 = s2 = load_cell(b, d1);  // NaN normal velocity: the second layer copies the first as it stands
+  } else {
+    s2 = load_cell(b, at(bc_source(kind, low, l, g2, false)));
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      if (kind == -80 || (kind == -50 && a == ax)) {
+        s1.w[1 + a] = -s1.w[1 + a];
+        s2.w[1 + a] = -s2.w[1 + a];
+      }
+    if (kind == -80) s2.p = s1.p;
+  }
+  store_cell(b, d1, s1);
+  store_cell(b, d2, s2);
 }
 
+// the ghost coordinate of a side (0 low, 1 high) and layer (0 inner)
+__device__ __forceinline__ int ghost_coord(int l, int side, int lay) { return side ? l + 1 + lay : 1 - lay; }
+
+// the ghost cells with two or three ghost axes
 template <typename T>
-__global__ void k_bc_pass(DevBlock<T> b, PhysParams P, int pass) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < bc_pass_items(b)) body_bc_pass(b, P, pass, t);
+__device__ __forceinline__ void body_bc_edge(const DevBlock<T>& b, const PhysParams& P, int t) {
+  const bool all = !bc_whole(b);  // with the corner cells' own ghost states
+  const int nc = all ? 16 : 12;
+  int i, j, k;
+  auto combo = [&](int q, int la, int lb, int& ca, int& cb) {
+    const int m = q % 3;
+    const int s = all ? q >> 2 : q / 3, l1 = all ? q & 1 : (m >= 1), l2 = all ? (q >> 1) & 1 : (m != 1);
+    ca = ghost_coord(la, s & 1, l1);
+    cb = ghost_coord(lb, s >> 1, l2);
+  };
+  if (t < nc * b.nz) {
+    combo(t / b.nz, b.il, b.jl, i, j);
+    k = 2 + t % b.nz;
+  } else if ((t -= nc * b.nz) < nc * b.ny) {
+    combo(t / b.ny, b.il, b.kl, i, k);
+    j = 2 + t % b.ny;
+  } else if ((t -= nc * b.ny) < nc * b.nx) {
+    combo(t / b.nx, b.jl, b.kl, j, k);
+    i = 2 + t % b.nx;
+  } else if ((t -= nc * b.nx) < 4 * nc) {
+    const int e = t & 3;
+    i = ghost_coord(b.il, e & 1, e >> 1);
+    combo(t >> 2, b.jl, b.kl, j, k);
+  } else {
+    i = j = k = 2;  // padding: a physical cell, not written
+  }
+  CellState<T> s;
+  if (ghost_state(b, P, i, j, k, s)) store_cell(b, cidx(b.Pi, b.Pj, i, j, k), s);
 }
 
-// bc_corner.f90:23-157: three dependent phases, each a set of independent
-// items (phase 0: edges along k and j, phase 1: edges along i, phase 2: the
-// eight corners); no item of a phase reads a cell another item of the same
-// phase writes
+// The corner cells of bc_corner.f90:23-157, after the faces: the inner edges
+// along k and j (k, j physical) from the two face ghosts beside them and the
+// physical cell, then those along i over the whole range, then the eight
+// corners from three such edge cells.  Four lanes share a cell: each takes
+// one of its terms, and lane 0 adds them up.  A corner's edge cells are formed
+// again from the face ghosts instead of waiting for the lanes that own them.
+// (0..ib, je, 1) is bc_corner.f90:120 as written, (x + a) - a; the corner
+// groups there also write the edge cell they read, because where the corner
+// cells run by themselves its ghost state is what is stored.
+// Every lane of a warp calls it.
 template <typename T>
-__device__ __forceinline__ int corner_items(const DevBlock<T>& b, int phase) {
-  return phase == 0 ? 4 * (b.kl - 1) + 4 * (b.jl - 1) : (phase == 1 ? 4 * (b.ib + 1) : 8);
-}
-
-template <typename T>
-__device__ void body_corner_item(const DevBlock<T>& b, const PhysParams& P, int phase, int t) {
-  const long long N = b.N;
+__device__ __forceinline__ void body_bc_corner(const DevBlock<T>& b, const PhysParams& P, int t) {
+  const int g0 = t >> 2, lane = t & 3;
   const int il = b.il, jl = b.jl, kl = b.kl, ie = b.ie, je = b.je, ke = b.ke;
+  const int n0 = 4 * b.nz, n1 = 4 * b.ny, n2 = 4 * (b.nx + 2);
+  int g = g0, kind = -1;  // 0: three-term edge, 1: (x + a) - a, 2: corner
+  int i = 2, j = 2, k = 2, ii = 2, jj = 2, kk = 2;  // the cell and the physical coordinates beside it
+  int a0 = 2, a1 = 2, a2 = 2;                       // this lane's term
+  if (g < n0) {
+    const int e = g / b.nz;
+    k = kk = 2 + g % b.nz;
+    i = e & 1 ? ie : 1, ii = e & 1 ? il : 2;
+    j = e >> 1 ? je : 1, jj = e >> 1 ? jl : 2;
+    kind = 0;
+    a0 = lane == 1 ? i : ii, a1 = lane == 0 ? j : jj, a2 = k;
+  } else if ((g -= n0) < n1) {
+    const int e = g / b.ny;
+    j = jj = 2 + g % b.ny;
+    i = e & 1 ? ie : 1, ii = e & 1 ? il : 2;
+    k = e >> 1 ? ke : 1, kk = e >> 1 ? kl : 2;
+    kind = 0;
+    a0 = lane == 1 ? i : ii, a1 = j, a2 = lane == 0 ? k : kk;
+  } else if ((g -= n1) < n2) {
+    const int e = g / (b.nx + 2), q = g % (b.nx + 2);
+    i = ii = q == 0 ? 0 : (q <= b.nx ? 1 + q : b.ib);
+    j = e & 1 ? je : 1, jj = e & 1 ? jl : 2;
+    k = e >> 1 ? ke : 1, kk = e >> 1 ? kl : 2;
+    kind = e == 1 ? 1 : 0;
+    a0 = i;
+    a1 = lane == (kind == 1 ? 0 : 1) ? j : jj;
+    a2 = lane == 0 ? k : kk;
+    // the cells next to a corner of that edge are written by the corner's group
+    if (kind == 1 && (i == 2 || i == il)) kind = -1;
+  } else if ((g -= n2) < 8) {
+    i = g & 1 ? ie : 1, ii = g & 1 ? il : 2;
+    j = (g >> 1) & 1 ? je : 1, jj = (g >> 1) & 1 ? jl : 2;
+    k = g >> 2 ? ke : 1, kk = g >> 2 ? kl : 2;
+    kind = 2;
+    a0 = lane == 2 ? i : ii;
+    a1 = lane == 1 || lane == 3 ? j : jj;
+    a2 = lane == 0 || lane == 3 ? k : kk;
+    if (lane == 3 && !(j == je && k == 1)) a1 = jj, a2 = kk;  // only that edge's own state is a term
+  }
+  CellState<T> s;
+  if (kind < 0 || (kind < 2 && lane == 3)) a0 = a1 = a2 = 2;  // no term: a physical cell
+  if (bc_whole(b))
+    ghost_state(b, P, a0, a1, a2, s);  // face ghosts and physical cells as stored
+  else
+    s = load_cell(b, cidx(b.Pi, b.Pj, a0, a1, a2));
+  T x[5], y[5], z[5], u[5];
+  const int lead = threadIdx.x & 28;
+#pragma unroll
+  for (int v = 0; v < 5; v++) {
+    x[v] = __shfl_sync(0xffffffffu, s.w[v], lead);
+    y[v] = __shfl_sync(0xffffffffu, s.w[v], lead + 1);
+    z[v] = __shfl_sync(0xffffffffu, s.w[v], lead + 2);
+    u[v] = __shfl_sync(0xffffffffu, s.w[v], lead + 3);
+  }
+  if (kind < 0 || lane != 0) return;
   const T gamma = (T)P.gamma;
-  auto C3 = [&](int i, int j, int k) { return cidx(b.Pi, b.Pj, i, j, k); };
-  auto set3 = [&](long long d, long long a, long long bb, long long cc) {
-    T wv[5];
+  CellState<T> o;
+  if (kind < 2) {
+#pragma unroll
+    for (int v = 0; v < 5; v++) o.w[v] = x[v] + y[v] - z[v];
+  } else {
+    const long long dq = cidx(b.Pi, b.Pj, ii, jj, kk);
+    const bool asis = j == je && k == 1;
+    CellState<T> e;
+#pragma unroll
     for (int v = 0; v < 5; v++) {
-      wv[v] = b.w[v * N + a] + b.w[v * N + bb] - b.w[v * N + cc];
-      b.w[v * N + d] = wv[v];
+      const T d = b.w[v * b.N + dq];
+      e.w[v] = asis ? u[v] + d - d : x[v] + y[v] - d;  // (ii, j, k)
+      const T bq = x[v] + z[v] - d;                     // (i, jj, k)
+      const T cq = y[v] + z[v] - d;                     // (i, j, kk)
+      o.w[v] = mdiv((e.w[v] + bq + cq) * T(2), T(3), T(1) / T(3)) - d;
     }
-    b.p[d] = depvars(gamma, wv);
-  };
-  if (phase == 0) {  // edges along k (k = 2..kl) and along j (j = 2..jl)
-    if (t < 4 * (kl - 1)) {
-      int k = 2 + t / 4, e = t % 4;
-      if (e == 0) set3(C3(1, 1, k), C3(2, 1, k), C3(1, 2, k), C3(2, 2, k));
-      else if (e == 1) set3(C3(ie, 1, k), C3(il, 1, k), C3(ie, 2, k), C3(il, 2, k));
-      else if (e == 2) set3(C3(1, je, k), C3(2, je, k), C3(1, jl, k), C3(2, jl, k));
-      else set3(C3(ie, je, k), C3(il, je, k), C3(ie, jl, k), C3(il, jl, k));
-    } else {
-      int u = t - 4 * (kl - 1);
-      int j = 2 + u / 4, e = u % 4;
-      if (e == 0) set3(C3(1, j, 1), C3(2, j, 1), C3(1, j, 2), C3(2, j, 2));
-      else if (e == 1) set3(C3(ie, j, 1), C3(il, j, 1), C3(ie, j, 2), C3(il, j, 2));
-      else if (e == 2) set3(C3(1, j, ke), C3(2, j, ke), C3(1, j, kl), C3(2, j, kl));
-      else set3(C3(ie, j, ke), C3(il, j, ke), C3(ie, j, kl), C3(il, j, kl));
+    if (asis) {
+      e.p = depvars_plain(gamma, e.w);
+      store_cell(b, cidx(b.Pi, b.Pj, ii, j, k), e);
     }
-  } else if (phase == 1) {  // edges along i (i = 0..ib)
-    int i = t / 4, e = t % 4;
-    if (e == 0) set3(C3(i, 1, 1), C3(i, 1, 2), C3(i, 2, 1), C3(i, 2, 2));
-    else if (e == 1) set3(C3(i, 1, ke), C3(i, 2, ke), C3(i, 1, kl), C3(i, 2, kl));
-    else if (e == 2) set3(C3(i, je, 1), C3(i, je, 1), C3(i, jl, 2), C3(i, jl, 2));  // bc_corner.f90:120 as written
-    else set3(C3(i, je, ke), C3(i, jl, ke), C3(i, je, kl), C3(i, jl, kl));
-  } else {  // the 8 corners; each reads only edge cells
-    long long d, a, bq, cq, dq;
-    switch (t) {
-      case 0: d = C3(1, 1, 1); a = C3(2, 1, 1); bq = C3(1, 2, 1); cq = C3(1, 1, 2); dq = C3(2, 2, 2); break;
-      case 1: d = C3(1, 1, ke); a = C3(2, 1, ke); bq = C3(1, 2, ke); cq = C3(1, 1, kl); dq = C3(2, 2, kl); break;
-      case 2: d = C3(1, je, 1); a = C3(2, je, 1); bq = C3(1, jl, 1); cq = C3(1, je, 2); dq = C3(2, jl, 2); break;
-      case 3: d = C3(ie, 1, 1); a = C3(il, 1, 1); bq = C3(ie, 2, 1); cq = C3(ie, 1, 2); dq = C3(il, 2, 2); break;
-      case 4: d = C3(ie, 1, ke); a = C3(il, 1, ke); bq = C3(ie, 2, ke); cq = C3(ie, 1, kl); dq = C3(il, 2, kl); break;
-      case 5: d = C3(ie, je, 1); a = C3(il, je, 1); bq = C3(ie, jl, 1); cq = C3(ie, je, 2); dq = C3(il, jl, 2); break;
-      case 6: d = C3(1, je, ke); a = C3(2, je, ke); bq = C3(1, jl, ke); cq = C3(1, je, kl); dq = C3(2, jl, kl); break;
-      default: d = C3(ie, je, ke); a = C3(il, je, ke); bq = C3(ie, jl, ke); cq = C3(ie, je, kl); dq = C3(il, jl, kl); break;
-    }
-    T wv[5];
-    for (int v = 0; v < 5; v++) {
-      wv[v] = (b.w[v * N + a] + b.w[v * N + bq] + b.w[v * N + cq]) * T(2) / T(3) - b.w[v * N + dq];
-      b.w[v * N + d] = wv[v];
-    }
-    b.p[d] = depvars(gamma, wv);
   }
+  o.p = depvars_plain(gamma, o.w);
+  store_cell(b, cidx(b.Pi, b.Pj, i, j, k), o);
 }
 
-
-template <typename T>
-__global__ void k_bc_corner(DevBlock<T> b, PhysParams P, int phase) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < corner_items(b, phase)) body_corner_item(b, P, phase, t);
+// part 0: the face ghosts; 1: the edge and corner ghosts; 2: the corner cells
+// of blocks with a face without a boundary condition
+template <typename T, int PART>
+__device__ __forceinline__ void body_bcond(const DevBlock<T>& b, const PhysParams& P, long long t) {
+  if (PART == 0) {
+    if (t < bc_n1(b)) body_bc_face(b, P, (int)t);
+  } else if (PART == 1) {
+    const int n2 = bc_n2(b);
+    if (t < n2)
+      body_bc_edge(b, P, (int)t);
+    else if (bc_whole(b) && t < (long long)n2 + bc_n3(b))
+      body_bc_corner(b, P, (int)t - n2);
+  } else {
+    if (!bc_whole(b) && t < bc_n3(b)) body_bc_corner(b, P, (int)t);
+  }
 }
-
-// the whole of bcond.f90 in one cooperative launch: the three face passes and
-// the three corner phases with a grid barrier between them
-template <typename T>
-__global__ void __launch_bounds__(256, 2) k_bcond_coop(DevBlock<T> b, PhysParams P) {
-  cg::grid_group g = cg::this_grid();
-  const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  const long long nf = bc_pass_items(b);
-  for (int pass = 0; pass < 3; pass++) {
-    for (long long t = gt; t < nf; t += gs) body_bc_pass(b, P, pass, t);
-    g.sync();
-  }
-  for (int phase = 0; phase < 3; phase++) {
-    const int n = corner_items(b, phase);
-    for (long long t = gt; t < n; t += gs) body_corner_item(b, P, phase, (int)t);
-    if (phase < 2) g.sync();
-  }
+template <typename T, int PART>
+__global__ void k_bcond(DevBlock<T> b, PhysParams P) {
+  body_bcond<T, PART>(b, P, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // --------------------------------------------------------------- residual norm (euler.f90:431-447)
@@ -2639,7 +2772,8 @@ __global__ void k_prim(DevBlock<T> b) {
   for (int a = 0; a < 3; a++) b.F[(long long)a * N + c] = mdiv(b.w[(long long)(1 + a) * N + c], r, y);
 }
 template <typename T>
-__global__ void __launch_bounds__(256, 4) k_face(DevBlock<T> b, PhysParams P, int dissip_on, T cd) {
+__global__ void __launch_bounds__(256, 4)
+    k_face(const __grid_constant__ DevBlock<T> b, const __grid_constant__ PhysParams P, int dissip_on, T cd) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL>(b, P, dissip_on, cd, t);
 }
@@ -2656,7 +2790,8 @@ __global__ void __launch_bounds__(256, 4) k_face_diss(DevBlock<T> b, PhysParams 
 }
 // the Roe faces (MUSCL states, upwind flux, and the viscous flux with NS)
 template <typename T>
-__global__ void __launch_bounds__(256, 3) k_face_roe(DevBlock<T> b, PhysParams P, int dissip_on, T cd) {
+__global__ void __launch_bounds__(256, 3)
+    k_face_roe(const __grid_constant__ DevBlock<T> b, const __grid_constant__ PhysParams P, int dissip_on, T cd) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_ROE>(b, P, dissip_on, cd, t);
 }
@@ -2806,14 +2941,15 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
     }
     for (long long t = gt; t < b.nmir; t += gs) body_cutcell(b, P, E.err, (int)t);
     g.sync();
-    for (int pass = 0; pass < 3; pass++) {
-      const long long nf = bc_pass_items(b);
-      for (long long t = gt; t < nf; t += gs) body_bc_pass(b, P, pass, t);
-      g.sync();
-    }
-    for (int phase = 0; phase < 3; phase++) {
-      const int n = corner_items(b, phase);
-      for (long long t = gt; t < n; t += gs) body_corner_item(b, P, phase, (int)t);
+    // whole warps of consecutive items: the corner cells share lanes
+    const long long lt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (long long t = lt; t < bc_n1(b); t += gs) body_bcond<T, 0>(b, P, t);
+    g.sync();
+    if (m < E.mstage && A.faces_only) continue;
+    for (long long t = lt; t < bc_n2(b) + (bc_whole(b) ? bc_n3(b) : 0); t += gs) body_bcond<T, 1>(b, P, t);
+    g.sync();
+    if (!bc_whole(b)) {
+      for (long long t = lt; t < bc_n3(b); t += gs) body_bcond<T, 2>(b, P, t);
       g.sync();
     }
   }
@@ -2956,16 +3092,9 @@ template <typename T> struct FCutcell {
     if (t < M.B[q].nmir) body_cutcell(M.B[q], M.P[q], M.err[q], (int)t);
   }
 };
-template <typename T> struct FBcPass {
-  int pass;
+template <typename T, int PART> struct FBcond {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t < bc_pass_items(M.B[q])) body_bc_pass(M.B[q], M.P[q], pass, t);
-  }
-};
-template <typename T> struct FCorner {
-  int phase;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t < corner_items(M.B[q], phase)) body_corner_item(M.B[q], M.P[q], phase, (int)t);
+    body_bcond<T, PART>(M.B[q], M.P[q], t);
   }
 };
 template <typename T> struct FDepvars {
@@ -3243,42 +3372,17 @@ void launch_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cu
 }
 
 template <typename T>
-void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s) {
-  const long long n = 2LL * ((long long)(b.jb + 1) * (b.kb + 1) + (long long)(b.ib + 1) * (b.kb + 1) +
-                             (long long)(b.ib + 1) * (b.jb + 1));
-  const int tpb = tpb_for(n);
-  // Six launches (three face passes, three corner phases) measured a little
-  // faster inside the cycle graphs than one cooperative launch with grid
-  // barriers; MGE_BCOND_COOP=1 selects the cooperative form (when every block
-  // it needs fits on the device at once; residency per block size).
-  static int resident[64][4] = {};
-  static int coop_env = -1;
-  if (coop_env < 0) {
-    const char* e = getenv("MGE_BCOND_COOP");
-    coop_env = (e && atoi(e) == 1) ? 1 : 0;
-  }
-  const int ti = tpb == 32 ? 0 : (tpb == 64 ? 1 : (tpb == 128 ? 2 : 3));
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (coop_env && dev >= 0 && dev < 64 && resident[dev][ti] == 0) {
-    int nsm = 0, per = 0, coop = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bcond_coop<T>, tpb, 0);
-    resident[dev][ti] = (coop && per > 0) ? nsm * per : -1;
-  }
-  const int grid = (coop_env && dev >= 0 && dev < 64) ? resident[dev][ti] : -1;
-  if (grid > 0) {
-    const int need = (int)std::max<long long>(1, std::min<long long>(nblk(n, tpb), grid));
-    DevBlock<T> bb = b;
-    PhysParams pp = P;
-    void* args[] = {&bb, &pp};
-    if (cudaLaunchCooperativeKernel((void*)k_bcond_coop<T>, need, tpb, args, 0, s) == cudaSuccess) return;
-    cudaGetLastError();
-  }
-  for (int pass = 0; pass < 3; pass++) k_bc_pass<T><<<LAUNCH_N(n), 0, s>>>(b, P, pass);
-  const long long nc = 4LL * (b.ib + b.jl + b.kl + 2);  // covers the items of phases 0 and 1
-  for (int phase = 0; phase < 3; phase++) k_bc_corner<T><<<LAUNCH_N(phase == 2 ? 8 : nc), 0, s>>>(b, P, phase);
+void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s, bool faces_only) {
+  k_bcond<T, 0><<<LAUNCH_N(bc_items_t(b, 0)), 0, s>>>(b, P);
+  if (faces_only) return;
+  k_bcond<T, 1><<<LAUNCH_N(bc_items_t(b, 1)), 0, s>>>(b, P);
+  const long long n = bc_items_t(b, 2);
+  if (n > 0) k_bcond<T, 2><<<LAUNCH_N(n), 0, s>>>(b, P);
+}
+
+template <typename T>
+long long bc_items(const DevBlock<T>& b, int part) {
+  return bc_items_t(b, part);
 }
 
 template <typename T>
@@ -3473,11 +3577,11 @@ static MultiArgs<T> multi_args(const MultiLevel& L) {
 }
 
 template <typename T>
-static void multi_bcond(const MultiLevel& L, MultiArgs<T>& M, cudaStream_t s) {
-  for (int pass = 0; pass < 3; pass++) go_multi(L, M, MK_BC, FBcPass<T>{pass}, s);
-  go_multi(L, M, MK_CORNER0, FCorner<T>{0}, s);
-  go_multi(L, M, MK_CORNER1, FCorner<T>{1}, s);
-  go_multi(L, M, MK_CORNER2, FCorner<T>{2}, s);
+static void multi_bcond(const MultiLevel& L, MultiArgs<T>& M, cudaStream_t s, bool faces_only = false) {
+  go_multi(L, M, MK_BC0, FBcond<T, 0>{}, s);
+  if (faces_only) return;
+  go_multi(L, M, MK_BC1, FBcond<T, 1>{}, s);
+  go_multi(L, M, MK_BC2, FBcond<T, 2>{}, s);
 }
 
 // timestep (optionally) and euler.f90:1-462 on one block of every case: the
@@ -3532,7 +3636,7 @@ static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, b
       go_multi(L, M, MK_PHYS, FUpdate<T>{a}, s);
     }
     go_multi(L, M, MK_REC, FCutcell<T>{}, s);
-    multi_bcond(L, M, s);
+    multi_bcond(L, M, s, a.faces_only && m < mstage);
   }
   if (rt) {
     go_multi(L, M, MK_RTP, FRtrmsPartial<T>{}, s);
@@ -3646,12 +3750,13 @@ __global__ void __launch_bounds__(256, 1) k_group_euler(MultiArgs<T> M, GroupEul
     }
     group_phase(M, G, MK_REC, FCutcell<T>{});
     grid.sync();
-    for (int pass = 0; pass < 3; pass++) {
-      group_phase(M, G, MK_BC, FBcPass<T>{pass});
-      grid.sync();
-    }
-    for (int phase = 0; phase < 3; phase++) {
-      group_phase(M, G, MK_CORNER0 + phase, FCorner<T>{phase});
+    group_phase(M, G, MK_BC0, FBcond<T, 0>{});
+    grid.sync();
+    if (a.faces_only && m < G.mstage) continue;
+    group_phase(M, G, MK_BC1, FBcond<T, 1>{});
+    grid.sync();
+    if (G.tot[MK_BC2] > 0) {
+      group_phase(M, G, MK_BC2, FBcond<T, 2>{});
       grid.sync();
     }
   }
@@ -3803,7 +3908,8 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   template void launch_irs<T>(const DevBlock<T>&, const PhysParams&, const IrsTables*, cudaStream_t, bool,       \
                               const int*, const StageArgs*);                                                    \
   template void launch_cutcell<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t);              \
-  template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                           \
+  template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t, bool);                     \
+  template long long bc_items<T>(const DevBlock<T>&, int);                                                      \
   template void launch_rtrms<T>(const DevBlock<T>&, const PhysParams&, int, double*, int, double*, cudaStream_t, \
                                 unsigned*);                                                                    \
   template void launch_depvars_all<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                     \

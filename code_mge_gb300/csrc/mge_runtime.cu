@@ -218,6 +218,18 @@ StageArgs stage_args(const mge_params& P, int m, int mgl, int mlvl, bool lres, b
   return A;
 }
 
+// Whether the edge and corner ghosts between two stages of an update are
+// dead: with a boundary condition on every face they are formed from the
+// physical cells alone, and the inviscid stages read face ghosts only (the
+// time step, the fluxes, the sensors and the wall terms all reach along one
+// axis).  The viscous gradients read edge ghosts, and so may a cut cell's
+// cloud.  The last stage always forms them.
+bool edges_dead(const mge_ctx* c, const Block& b) {
+  for (int f = 0; f < 6; f++)
+    if (b.bctype[f] == 0) return false;
+  return c->prm.eqntype == MGE_EQN_EULER && (b.recs.empty() || b.cut_beside_bcond);
+}
+
 // timestep.f90 (optionally) followed by euler.f90:1-462 on one block;
 // nstage_limit > 0 stops after that stage (parity probes)
 void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir, int nstage_limit, bool rt,
@@ -237,6 +249,7 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
     for (int m = 1; m <= mstage; m++) {
       L.st[m - 1] = stage_args(P, m, mgl, mlvl, lres, lfir, itime);
       L.st[m - 1].fast = b.fast;
+      L.st[m - 1].faces_only = edges_dead(c, b);
     }
     for (int d = 0; d < 3; d++) L.tab[d] = b.tabs[d];
     L.rt_partial = b.rt_partial;
@@ -279,6 +292,8 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
     for (int m = 1; m <= mstage; m++) {
       StageArgs A = stage_args(P, m, mgl, mlvl, lres, lfir, itime);
       A.fast = b.fast;
+      A.faces_only = edges_dead(c, b);
+      const bool faces_only = A.faces_only && m < mstage;
       launch_stage<T>(D, c->P, A, c->d_err, c->stream, c->side, c->ev_fork, c->ev_join);
       if (lres) return;
       if (A.irs) launch_irs<T>(D, c->P, b.tabs, c->stream, b.aux32, b.irs_var, &A);
@@ -287,11 +302,11 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
         cudaStreamWaitEvent(c->side, c->ev_fork, 0);
         launch_cutcell<T>(D, c->P, c->d_err, c->side);
         cudaEventRecord(c->ev_join, c->side);
-        launch_bcond<T>(D, c->P, c->stream);
+        launch_bcond<T>(D, c->P, c->stream, faces_only);
         cudaStreamWaitEvent(c->stream, c->ev_join, 0);
       } else {
         launch_cutcell<T>(D, c->P, c->d_err, c->stream);
-        launch_bcond<T>(D, c->P, c->stream);
+        launch_bcond<T>(D, c->P, c->stream, faces_only);
       }
     }
     if (want_rt) launch_rtrms<T>(D, c->P, P.vt, b.rt_partial, b.npart, b.rt_cur, c->stream, c->d_err);
@@ -1795,7 +1810,13 @@ int mge_kernel_times(mge_ctx* c, int level, int reps, double* ms_out, int nout) 
             });
           });
       if (!rc) rc = timed(8, [&] { enqueue_simple(c, b, 4); });
-      if (!rc) rc = timed(9, [&] { enqueue_simple(c, b, 2); });
+      if (!rc)
+        rc = timed(9, [&] {
+          with_dev(b, [&](auto& D) {
+            using T = typename std::remove_reference_t<decltype(D)>::value_type;
+            launch_bcond<T>(D, c->P, c->stream, edges_dead(c, b) && m < P.mstage);
+          });
+        });
     }
     if (!rc)
       rc = timed(10, [&] {
@@ -1944,11 +1965,7 @@ void kind_counts(const Block& b, long long* n) {
   n[MK_IRS0] = 5 * ny * nz;
   n[MK_IRS1] = 5 * nx * nz;
   n[MK_IRS2] = 5 * nx * ny;
-  n[MK_BC] = 2 * ((long long)(b.jb + 1) * (b.kb + 1) + (long long)(b.ib + 1) * (b.kb + 1) +
-                  (long long)(b.ib + 1) * (b.jb + 1));
-  n[MK_CORNER0] = 4LL * (b.kl - 1) + 4LL * (b.jl - 1);
-  n[MK_CORNER1] = 4LL * (b.ib + 1);
-  n[MK_CORNER2] = 8;
+  for (int q = 0; q < 3; q++) n[MK_BC0 + q] = b.f32 ? bc_items(b.dev32, q) : bc_items(b.dev, q);
   n[MK_RTP] = 256LL * b.npart;
   n[MK_ONE] = 1;
 }
@@ -2116,6 +2133,8 @@ void group_euler(GroupPlan& G, int level, int mgl, int mlvl, bool lres, bool lfi
   for (int m = 1; m <= P.mstage; m++) {
     A[m - 1] = stage_args(P, m, mgl, mlvl, lres, lfir, 0);
     A[m - 1].fast = G.lv[level - 1].fast;
+    A[m - 1].faces_only = 1;
+    for (mge_ctx* c : G.cases) A[m - 1].faces_only &= edges_dead(c, c->lv[level - 1][0]);
   }
   multi_euler(G.lv[level - 1], A, P.mstage, with_timestep, lfir, rt && !lres, G.stream);
 }
