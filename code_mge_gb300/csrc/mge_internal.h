@@ -157,6 +157,8 @@ enum MultiKind {
   MK_PHYS = 0,   // physical cells nx*ny*nz
   MK_PREP,       // [1..ie]^3
   MK_FACE,       // [2..ie]^3
+  MK_PREP3,      // the prep pass in three rows, one per direction
+  MK_FACE3,      // the face pass in three rows
   MK_N,          // all cells N
   MK_N5,         // 5N
   MK_REC,        // cut-cell records
@@ -175,6 +177,7 @@ enum MultiKind {
 struct MultiLevel {
   int nc = 0;
   bool f32 = false, aux32 = false, fast = false;
+  bool prep_rows = false, face_rows = false;  // the passes that run in rows
   bool coop = false;             // the update as one persistent cooperative launch (k_group_euler)
   void* B = nullptr;             // DevBlock<T>[nc]
   PhysParams* P = nullptr;       // [nc]
@@ -236,6 +239,10 @@ template <typename T> void launch_bcond(const DevBlock<T>& b, const PhysParams& 
                                         bool faces_only = false);
 // work items of the boundary launches (part 0, 1, 2; 0 items: no launch)
 template <typename T> long long bc_items(const DevBlock<T>& b, int part);
+// items of the prep (e = 2) or face (e = 1) pass in rows, and which of the two
+// a level of so many cells runs so
+template <typename T> long long split_items(const DevBlock<T>& b, int e);
+void split_passes(const PhysParams& P, bool fast, long long cells, bool* prep, bool* face);
 template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* partial,
                                         int npartial, double* out, cudaStream_t s, unsigned* err = nullptr);
 template <typename T> void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);

@@ -70,6 +70,29 @@ __device__ __forceinline__ double smdiv(double a, double b, double y) {
   return fma(r, y, q);
 }
 __device__ __forceinline__ float smdiv(float a, float b, float y) { return mdiv(a, b, y); }
+// the same by choice: S takes the integer pipes.  They win where a kernel is
+// bound by the FP64 rate; a level of few cells is bound by the latency of its
+// dependent chains, and there the plain operations are the shorter ones (a
+// product 32 cycles against about 100).  The bits are the same either way.
+template <bool S, typename T> __device__ __forceinline__ T pmul(T a, T b) {
+  if constexpr (S) return smul(a, b); else return a * b;
+}
+template <bool S, typename T> __device__ __forceinline__ T pdiv(T a, T b) {
+  if constexpr (S) return sdiv(a, b); else return a / b;
+}
+template <bool S, typename T> __device__ __forceinline__ T pmdiv(T a, T b, T y) {
+  if constexpr (S) return smdiv(a, b, y); else return mdiv(a, b, y);
+}
+// cell (or face) t of a box of nx by ny by any number of cells, counted from
+// (i0, i0, i0).  A block's scratch alone holds 64 fields, so its cells number
+// fewer than 2^31 on any device and 32-bit divisions suffice (a 64-bit one
+// costs about ten times as much).
+__device__ __forceinline__ void cell_of(long long t, int nx, int ny, int i0, int& i, int& j, int& k) {
+  const unsigned u = (unsigned)t, q = u / (unsigned)nx, r = q / (unsigned)ny;
+  i = i0 + (int)(u - q * (unsigned)nx);
+  j = i0 + (int)(q - r * (unsigned)ny);
+  k = i0 + (int)r;
+}
 // reciprocals the host prepares once, RN(1/x) of the divisor x in the
 // block's precision, so that mdiv gives the correctly rounded quotient
 __device__ __forceinline__ double rcp_gm1(const PhysParams& P, double) { return P.rgm1; }
@@ -95,11 +118,11 @@ template <typename T> __device__ __forceinline__ T fmaxT(T a, T b) { return a > 
 template <typename T> __device__ __forceinline__ T fminT(T a, T b) { return a < b ? a : b; }
 
 // depvars_one, depvars.f90:48-49
-template <typename T> __device__ __forceinline__ T depvars(T gamma, const T* w) {
+template <bool S = true, typename T = double> __device__ __forceinline__ T depvars(T gamma, const T* w) {
   // the products on the integer pipes and the halving as an exponent step:
   // the same bits as 0.5*(w1*w1 + w2*w2 + w3*w3)/w0 and (gamma-1)*dim(w4, qq)
-  T qq = sdiv(mulhalf(smul(w[1], w[1]) + smul(w[2], w[2]) + smul(w[3], w[3])), w[0]);
-  return smul(gamma - T(1), fdimT(w[4], qq));
+  T qq = pdiv<S>(mulhalf(pmul<S>(w[1], w[1]) + pmul<S>(w[2], w[2]) + pmul<S>(w[3], w[3])), w[0]);
+  return pmul<S>(gamma - T(1), fdimT(w[4], qq));
 }
 
 struct Idx {
@@ -113,44 +136,43 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 // --------------------------------------------------------------- timestep (timestep.f90:39-115)
 // TC is the arithmetic precision (FP64 in the plain path, FP32 in the mixed one).
-template <typename T, typename TC>
+template <typename T, typename TC, bool S = true>
 __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err,
                                                             long long t) {
   const int nxl = b.nx, nyl = b.ny;
   unsigned long long mine = ~0ull;  // bits of this cell's vdtim for the global minimum
-  int i = 2 + (int)(t % nxl);
-  int j = 2 + (int)((t / nxl) % nyl);
-  int k = 2 + (int)(t / ((long long)nxl * nyl));
+  int i, j, k;
+  cell_of(t, nxl, nyl, 2, i, j, k);
   const long long N = b.N;
   const long long c = cidx(b.Pi, b.Pj, i, j, k);
   const TC gamma = (TC)P.gamma;
   TC w0 = (TC)b.w[c], w1 = (TC)b.w[N + c], w2 = (TC)b.w[2 * N + c], w3 = (TC)b.w[3 * N + c];
   TC pc = (TC)b.p[c];
-  TC y = sdiv(TC(1), w0);
-  TC cc = smdiv(smul(gamma, pc), w0, y);
+  TC y = pdiv<S>(TC(1), w0);
+  TC cc = pmdiv<S>(pmul<S>(gamma, pc), w0, y);
   if (cc < TC(0) || cc != cc) {  // timestep.f90:45-48
     atomicCAS(err, 0u, (unsigned)ERR_NEGPRESS);  // the first stop in launch order wins
     return mine;
   }
   cc = sqrt(fmaxT(cc, TC(0)));
-  TC uu = smdiv(w1, w0, y), uv = smdiv(w2, w0, y), uw = smdiv(w3, w0, y);
+  TC uu = pmdiv<S>(w1, w0, y), uv = pmdiv<S>(w2, w0, y), uw = pmdiv<S>(w3, w0, y);
   // face vectors are axis-aligned: |u.s| = |u_d s_d|, |s| precomputed
-  TC ri = fabs(smul(uu, (TC)b.s[0])) + smul(cc, (TC)b.sqrt_ds[0]);
-  TC rj = fabs(smul(uv, (TC)b.s[1])) + smul(cc, (TC)b.sqrt_ds[1]);
-  TC rk = fabs(smul(uw, (TC)b.s[2])) + smul(cc, (TC)b.sqrt_ds[2]);
+  TC ri = fabs(pmul<S>(uu, (TC)b.s[0])) + pmul<S>(cc, (TC)b.sqrt_ds[0]);
+  TC rj = fabs(pmul<S>(uv, (TC)b.s[1])) + pmul<S>(cc, (TC)b.sqrt_ds[1]);
+  TC rk = fabs(pmul<S>(uw, (TC)b.s[2])) + pmul<S>(cc, (TC)b.sqrt_ds[2]);
   TC lsum = ri + rj + rk;
   TC fict;
   if (P.eqn_ns) {  // viscous spectral radii, timestep.f90:141-178
-    const TC fmue = sdiv((TC)P.viscl, (TC)P.prlmean);
-    const TC f1 = sdiv(sdiv(TC(4), w0), TC(3));
-    const TC f2 = sdiv(gamma, w0);
+    const TC fmue = pdiv<S>((TC)P.viscl, (TC)P.prlmean);
+    const TC f1 = pdiv<S>(pdiv<S>(TC(4), w0), TC(3));
+    const TC f2 = pdiv<S>(gamma, w0);
     const TC fac = fmaxT(f1, f2);
-    const TC dtv = sdiv(fac * fmue, (TC)b.vol);
+    const TC dtv = pdiv<S>(fac * fmue, (TC)b.vol);
     const TC s0 = (TC)b.s[0], s1 = (TC)b.s[1], s2 = (TC)b.s[2];
     TC rvi = dtv * (s0 * s0), rvj = dtv * (s1 * s1), rvk = dtv * (s2 * s2);
-    fict = sdiv((TC)b.vol, lsum + (TC)P.cfac * (rvi + rvj + rvk));
+    fict = pdiv<S>((TC)b.vol, lsum + (TC)P.cfac * (rvi + rvj + rvk));
   } else {
-    fict = sdiv((TC)b.vol, lsum);
+    fict = pdiv<S>((TC)b.vol, lsum);
   }
   const TC plim = TC(0.001);
   TC pip = (TC)b.p[c + 1], pim = (TC)b.p[c - 1];
@@ -158,15 +180,15 @@ __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b
   long long pl = (long long)b.Pi * b.Pj;
   TC pkp = (TC)b.p[c + pl], pkm = (TC)b.p[c - pl];
   TC p2 = mul2(pc);
-  TC dpi = fabs(sdiv(pip - p2 + pim, pip + p2 + pim + plim));
-  TC dpj = fabs(sdiv(pjp - p2 + pjm, pjp + p2 + pjm + plim));
-  TC dpk = fabs(sdiv(pkp - p2 + pkm, pkp + p2 + pkm + plim));
-  TC r = sdiv(TC(1), TC(1) + fminT((TC)P.dimcfl, mul2(dpi + dpj + dpk)));
+  TC dpi = fabs(pdiv<S>(pip - p2 + pim, pip + p2 + pim + plim));
+  TC dpj = fabs(pdiv<S>(pjp - p2 + pjm, pjp + p2 + pjm + plim));
+  TC dpk = fabs(pdiv<S>(pkp - p2 + pkm, pkp + p2 + pkm + plim));
+  TC r = pdiv<S>(TC(1), TC(1) + fminT((TC)P.dimcfl, mul2(dpi + dpj + dpk)));
   if (P.unsteady) {  // timestep.f90:85-99,180-190: at most 2*dtstep/(3*cfl)
     const TC dtime = (TC(2) * (TC)P.dtstep) / (TC(3) * (TC)P.cfl);
     fict = fict < dtime ? fict : dtime;
   }
-  TC vd = smul(fict, r);
+  TC vd = pmul<S>(fict, r);
   double vdd = (double)vd;
   if (vdd >= 0.0) mine = (unsigned long long)__double_as_longlong(vdd);
   if (b.blank[c] == 0) {  // timestep.f90:212-223
@@ -221,11 +243,11 @@ __device__ __forceinline__ void block_min_to(unsigned long long mine, double* dt
   }
 }
 
-template <typename T, typename TC>
+template <typename T, typename TC, bool S>
 __global__ void k_timestep(DevBlock<T> b, PhysParams P, unsigned* err) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long mine = ~0ull;
-  if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC>(b, P, err, t);
+  if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC, S>(b, P, err, t);
   block_min_to(mine, b.dtim);  // global dtim (timestep.f90:112), kept even when vt = 0
 }
 
@@ -256,26 +278,25 @@ __device__ __forceinline__ T van_albada(T a, T b, T e2);
 // once and multiplies, F(v) = q w(v), instead of rounding each product
 // before its division.  The result is the same quantity to an FP64 rounding
 // or two, not the reference's bit pattern.
-template <typename T, bool SLOPES = false, bool FAST = false>
+template <typename T, bool SLOPES = false, bool FAST = false, bool S = true>
 __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams& P, int dissip_on, long long t) {
   const int ex = b.ie, ey = b.je;  // count = ie (cells 1..ie)
-  int i = 1 + (int)(t % ex);
-  int j = 1 + (int)((t / ex) % ey);
-  int k = 1 + (int)(t / ((long long)ex * ey));
+  int i, j, k;
+  cell_of(t, ex, ey, 1, i, j, k);
   const long long N = b.N;
   const long long c = cidx(b.Pi, b.Pj, i, j, k);
   T w[5];
 #pragma unroll
   for (int v = 0; v < 5; v++) w[v] = b.w[v * N + c];
   T p = b.p[c];
-  T y = sdiv(T(1), w[0]);
+  T y = pdiv<S>(T(1), w[0]);
   T Hc = w[4] + p;
   b.H[c] = Hc;
   if (P.eqn_ns && dissip_on) {  // velocity and temperature, zero in solid cells (euler.f90:140-154)
     const bool solid = b.blank[c] == 0;
 #pragma unroll
     for (int a = 0; a < 3; a++) b.vt[a * N + c] = solid ? T(0) : mdiv(w[1 + a], w[0], y);
-    b.vt[3 * N + c] = solid ? T(0) : sdiv(p, w[0] * (T)P.gas_const);
+    b.vt[3 * N + c] = solid ? T(0) : pdiv<S>(p, w[0] * (T)P.gas_const);
   }
   if (SLOPES) {
     const long long sts[3] = {1, (long long)b.Pi, (long long)b.Pi * b.Pj};
@@ -303,9 +324,9 @@ __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       const T s = (T)b.s[d];
-      const T f0 = smul(w[1 + d], s);
-      const T q = smul(f0, y);
-      T f1 = smul(q, w[1]), f2 = smul(q, w[2]), f3 = smul(q, w[3]);
+      const T f0 = pmul<S>(w[1 + d], s);
+      const T q = pmul<S>(f0, y);
+      T f1 = pmul<S>(q, w[1]), f2 = pmul<S>(q, w[2]), f3 = pmul<S>(q, w[3]);
       if (d == 0) f1 = fma(p, s, f1);
       if (d == 1) f2 = fma(p, s, f2);
       if (d == 2) f3 = fma(p, s, f3);
@@ -314,7 +335,7 @@ __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams
       F[N] = f1;
       F[2 * N] = f2;
       F[3 * N] = f3;
-      F[4 * N] = smul(q, Hc);
+      F[4 * N] = pmul<S>(q, Hc);
     }
   } else if (P.distype != 2) {
 #pragma unroll
@@ -322,14 +343,14 @@ __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams
       // the products of this FP64-bound pass go to the integer pipes (smul);
       // the fused steps of the quotients stay on the FP64 pipe
       T s = (T)b.s[d];
-      T f0 = smul(w[1 + d], s);  // sum(w(2:4)*ss) with the two zero components dropped
-      T f1 = smdiv(smul(f0, w[1]), w[0], y);
-      T f2 = smdiv(smul(f0, w[2]), w[0], y);
-      T f3 = smdiv(smul(f0, w[3]), w[0], y);
-      if (d == 0) f1 = f1 + smul(p, s);
-      if (d == 1) f2 = f2 + smul(p, s);
-      if (d == 2) f3 = f3 + smul(p, s);
-      T f4 = smdiv(smul(f0, Hc), w[0], y);
+      T f0 = pmul<S>(w[1 + d], s);  // sum(w(2:4)*ss) with the two zero components dropped
+      T f1 = pmdiv<S>(pmul<S>(f0, w[1]), w[0], y);
+      T f2 = pmdiv<S>(pmul<S>(f0, w[2]), w[0], y);
+      T f3 = pmdiv<S>(pmul<S>(f0, w[3]), w[0], y);
+      if (d == 0) f1 = f1 + pmul<S>(p, s);
+      if (d == 1) f2 = f2 + pmul<S>(p, s);
+      if (d == 2) f3 = f3 + pmul<S>(p, s);
+      T f4 = pmdiv<S>(pmul<S>(f0, Hc), w[0], y);
       T* F = b.F + (long long)(d * 5) * N + c;
       F[0] = f0;
       F[N] = f1;
@@ -358,21 +379,78 @@ __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams
     {
       T pm = b.p[c - 1], pp = b.p[c + 1], p2 = mul2(p);
       T pb = fabs(pm + p2 + pp);
-      b.fp[c] = (pb > T(0)) ? sdiv(fabs(pm - p2 + pp), pb) : T(0);
+      b.fp[c] = (pb > T(0)) ? pdiv<S>(fabs(pm - p2 + pp), pb) : T(0);
     }
     // j: abs(p(j+1) +2p(j) +p(j-1)), dflux.f90:131-136
     {
       T pm = b.p[c - b.Pi], pp = b.p[c + b.Pi], p2 = mul2(p);
       T pb = fabs(pp + p2 + pm);
-      b.fp[N + c] = (pb > T(0)) ? sdiv(fabs(pp - p2 + pm), pb) : T(0);
+      b.fp[N + c] = (pb > T(0)) ? pdiv<S>(fabs(pp - p2 + pm), pb) : T(0);
     }
     // k: abs(p(k-1) +2p(k) +p(k+1)), dflux.f90:188-193
     {
       T pm = b.p[c - pl], pp = b.p[c + pl], p2 = mul2(p);
       T pb = fabs(pm + p2 + pp);
-      b.fp[2 * N + c] = (pb > T(0)) ? sdiv(fabs(pm - p2 + pp), pb) : T(0);
+      b.fp[2 * N + c] = (pb > T(0)) ? pdiv<S>(fabs(pm - p2 + pp), pb) : T(0);
     }
   }
+}
+
+// One direction of the prep pass for the central scheme of the Euler
+// equations: the cell flux, the differences and the sensor along D, at the
+// cells a face along D reads (tangential indices physical).  Three times the
+// threads of body_prep with a third of its chain each, for the levels that
+// leave most of the chip idle.
+template <typename T, bool FAST, bool S, int D>
+__device__ __forceinline__ void body_prep_dir(const DevBlock<T>& b, const PhysParams& P, int dissip_on, int t) {
+  const int n0 = b.nx + (D == 0 ? 2 : 0), n1 = b.ny + (D == 1 ? 2 : 0), n2 = b.nz + (D == 2 ? 2 : 0);
+  if (t >= n0 * n1 * n2) return;
+  int i, j, k;
+  cell_of(t, n0, n1, 2, i, j, k);
+  if (D == 0) i -= 1;
+  if (D == 1) j -= 1;
+  if (D == 2) k -= 1;
+  const long long N = b.N, st = D == 0 ? 1 : (D == 1 ? (long long)b.Pi : (long long)b.Pi * b.Pj);
+  const long long c = cidx(b.Pi, b.Pj, i, j, k);
+  T w[5], wn[5], p = b.p[c], pm = T(0), pp = T(0);
+#pragma unroll
+  for (int v = 0; v < 5; v++) w[v] = b.w[v * N + c];
+  if (dissip_on) {
+#pragma unroll
+    for (int v = 0; v < 5; v++) wn[v] = b.w[v * N + c - st];
+    pm = b.p[c - st], pp = b.p[c + st];
+  }
+  const T y = pdiv<S>(T(1), w[0]), Hc = w[4] + p;
+  if (P.matrix) b.H[c] = Hc;
+  const T s = (T)b.s[D];
+  const T f0 = pmul<S>(w[1 + D], s);
+  T f[5];
+  f[0] = f0;
+  if (FAST) {
+    const T q = pmul<S>(f0, y);
+#pragma unroll
+    for (int v = 1; v < 4; v++) f[v] = v == 1 + D ? fma(p, s, pmul<S>(q, w[v])) : pmul<S>(q, w[v]);
+    f[4] = pmul<S>(q, Hc);
+  } else {
+#pragma unroll
+    for (int v = 1; v < 4; v++) {
+      f[v] = pmdiv<S>(pmul<S>(f0, w[v]), w[0], y);
+      if (v == 1 + D) f[v] = f[v] + pmul<S>(p, s);
+    }
+    f[4] = pmdiv<S>(pmul<S>(f0, Hc), w[0], y);
+  }
+  T* F = b.F + (long long)(D * 5) * N + c;
+#pragma unroll
+  for (int v = 0; v < 5; v++) F[v * N] = f[v];
+  if (!dissip_on) return;
+  T* Dl = b.dlt + (long long)(D * 5) * N + c;
+#pragma unroll
+  for (int v = 0; v < 4; v++) Dl[v * N] = w[v] - wn[v];
+  Dl[4 * N] = Hc - (wn[4] + pm);
+  const T p2 = mul2(p);
+  const T pb = D == 1 ? fabs(pp + p2 + pm) : fabs(pm + p2 + pp);
+  const T pa = D == 1 ? fabs(pp - p2 + pm) : fabs(pm - p2 + pp);
+  b.fp[D * N + c] = (pb > T(0)) ? pdiv<S>(pa, pb) : T(0);
 }
 
 // dflux_matrix, dflux.f90:283-339, with general face vector ss
@@ -610,7 +688,7 @@ __device__ __noinline__ void visc_face(const DevBlock<T>& b, const PhysParams& P
 // the central scheme with scalar dissipation and no viscous flux, without
 // the registers the matrix dissipation and the viscous face would take.
 enum { FACE_CENTRAL = 0, FACE_ROE = 1, FACE_ANY = 2, FACE_JST = 3 };
-template <typename T, int D, int SCH>
+template <typename T, int D, int SCH, bool S>
 __device__ __forceinline__ void face_dir(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd, int i, int j,
                                          int k) {
   const long long N = b.N;
@@ -634,7 +712,7 @@ __device__ __forceinline__ void face_dir(const DevBlock<T>& b, const PhysParams&
       face_states_pre<T, D>(b, P, c, q, wl, &pl, wr, &pr);
     else
       face_states<T, D>(b, P, c, q, P.distype == 2 ? 2 : 1, wl, &pl, wr, &pr);
-    const T yl = sdiv(T(1), wl[0]), yr = sdiv(T(1), wr[0]);
+    const T yl = pdiv<S>(T(1), wl[0]), yr = pdiv<S>(T(1), wr[0]);
     if (P.distype == 2) {
       T f1[5], f2[5];
       ceflux_gen<T>(D, wr, pr, (T)b.s[D], yr, f1);
@@ -687,11 +765,11 @@ __device__ __forceinline__ void face_dir(const DevBlock<T>& b, const PhysParams&
     T dm = (q - 1 == 1) ? d0 : Dl[v * N + c - st];
     T dp = (q + 1 == bq) ? d0 : Dl[v * N + c + st];
     T t3 = dp - mul2(d0) + dm;
-    out[v] = smul(dis2, d0) - smul(dis4, t3);
+    out[v] = pmul<S>(dis2, d0) - pmul<S>(dis4, t3);
   }
   if (SCH == FACE_JST || !P.matrix) {
 #pragma unroll
-    for (int v = 0; v < 5; v++) out[v] = smul(out[v], lam);
+    for (int v = 0; v < 5; v++) out[v] = pmul<S>(out[v], lam);
   } else {
     T ss[3] = {T(0), T(0), T(0)};
     ss[D] = (T)b.s[D];
@@ -713,23 +791,22 @@ __device__ __forceinline__ void face_dir(const DevBlock<T>& b, const PhysParams&
   (void)eq;
 }
 
-template <typename T, int SCH = FACE_ANY>
+template <typename T, int SCH = FACE_ANY, bool S = true>
 __device__ __forceinline__ void body_face(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd, long long t) {
   const int ex = b.ie - 1, ey = b.je - 1;  // 2..ie
-  int i = 2 + (int)(t % ex);
-  int j = 2 + (int)((t / ex) % ey);
-  int k = 2 + (int)(t / ((long long)ex * ey));
+  int i, j, k;
+  cell_of(t, ex, ey, 2, i, j, k);
   bool jp = j <= b.jl, kp = k <= b.kl, ip = i <= b.il;
-  if (jp && kp) face_dir<T, 0, SCH>(b, P, dissip_on, cd, i, j, k);
-  if (ip && kp) face_dir<T, 1, SCH>(b, P, dissip_on, cd, i, j, k);
-  if (ip && jp) face_dir<T, 2, SCH>(b, P, dissip_on, cd, i, j, k);
+  if (jp && kp) face_dir<T, 0, SCH, S>(b, P, dissip_on, cd, i, j, k);
+  if (ip && kp) face_dir<T, 1, SCH, S>(b, P, dissip_on, cd, i, j, k);
+  if (ip && jp) face_dir<T, 2, SCH, S>(b, P, dissip_on, cd, i, j, k);
 }
 
 // The contracted form's dissipation face (scalar JST, dflux.f90:87-112): the
 // combine pass forms the convective part from the cell fluxes, so only dfs is
 // written.  The face's coefficients take lambda once, dis2*lambda and
 // dis4*lambda, and each variable is one product and two multiply-adds.
-template <typename T, int D>
+template <typename T, int D, bool S>
 __device__ __forceinline__ void face_diss_fast(const DevBlock<T>& b, const PhysParams& P, T cd, int i, int j, int k) {
   const long long N = b.N;
   const long long st = D == 0 ? 1 : (D == 1 ? (long long)b.Pi : (long long)b.Pi * b.Pj);
@@ -744,9 +821,9 @@ __device__ __forceinline__ void face_diss_fast(const DevBlock<T>& b, const PhysP
   const long long cm = (q - 1 < 2) ? c : c - st;
   const long long cp = (q > lq) ? c - st : c;
   const T lam = mulhalf(b.lam[cm] + b.lam[cp]);
-  const T dis2 = smul((T)P.vis2, ep);
+  const T dis2 = pmul<S>((T)P.vis2, ep);
   const T dis4 = gt_nonneg((T)P.vis4, dis2) ? (T)P.vis4 - dis2 : T(0);
-  const T a2 = smul(smul(dis2, cd), lam), a4 = smul(smul(dis4, cd), lam);
+  const T a2 = pmul<S>(pmul<S>(dis2, cd), lam), a4 = pmul<S>(pmul<S>(dis4, cd), lam);
   const T* Dl = b.dlt + (long long)(D * 5) * N;
   T* Df = b.dfs + (long long)(D * 5) * N;
 #pragma unroll
@@ -755,20 +832,48 @@ __device__ __forceinline__ void face_diss_fast(const DevBlock<T>& b, const PhysP
     const T dm = (q - 1 == 1) ? d0 : Dl[v * N + c - st];
     const T dp = (q + 1 == bq) ? d0 : Dl[v * N + c + st];
     const T t3 = fma(T(-2), d0, dp + dm);
-    Df[v * N + c] = fma(a2, d0, -smul(a4, t3));
+    Df[v * N + c] = fma(a2, d0, -pmul<S>(a4, t3));
   }
 }
 
+// One direction of the face pass, at the faces along D between physical lines
+// of cells; FAST: the contracted form's dissipation faces
+template <typename T, bool FAST, bool S, int D>
+__device__ __forceinline__ void body_face_split(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd, int t) {
+  const int n0 = b.nx + (D == 0), n1 = b.ny + (D == 1), n2 = b.nz + (D == 2);
+  if (t >= n0 * n1 * n2) return;
+  int i, j, k;
+  cell_of(t, n0, n1, 2, i, j, k);
+  if (FAST)
+    face_diss_fast<T, D, S>(b, P, cd, i, j, k);
+  else
+    face_dir<T, D, FACE_JST, S>(b, P, dissip_on, cd, i, j, k);
+}
+
+// The split passes as one range of items: three rows, one per direction, each
+// of whole 256-thread blocks (e = 2: prep, 1: faces)
 template <typename T>
-__device__ __forceinline__ void body_face_diss(const DevBlock<T>& b, const PhysParams& P, T cd, long long t) {
-  const int ex = b.ie - 1, ey = b.je - 1;  // 2..ie
-  int i = 2 + (int)(t % ex);
-  int j = 2 + (int)((t / ex) % ey);
-  int k = 2 + (int)(t / ((long long)ex * ey));
-  bool jp = j <= b.jl, kp = k <= b.kl, ip = i <= b.il;
-  if (jp && kp) face_diss_fast<T, 0>(b, P, cd, i, j, k);
-  if (ip && kp) face_diss_fast<T, 1>(b, P, cd, i, j, k);
-  if (ip && jp) face_diss_fast<T, 2>(b, P, cd, i, j, k);
+__host__ __device__ __forceinline__ long long split_row(const DevBlock<T>& b, int e) {
+  const long long x = (long long)(b.nx + e) * b.ny * b.nz, y = (long long)b.nx * (b.ny + e) * b.nz,
+                  z = (long long)b.nx * b.ny * (b.nz + e);
+  const long long m = x > y ? (x > z ? x : z) : (y > z ? y : z);
+  return (m + 255) / 256 * 256;
+}
+template <typename T> long long split_items_t(const DevBlock<T>& b, int e) { return 3 * split_row(b, e); }
+template <typename T, bool FAST, bool S>
+__device__ __forceinline__ void body_prep_rows(const DevBlock<T>& b, const PhysParams& P, int dissip_on, long long t) {
+  const long long row = split_row(b, 2);
+  if (t < row) body_prep_dir<T, FAST, S, 0>(b, P, dissip_on, (int)t);
+  else if (t < 2 * row) body_prep_dir<T, FAST, S, 1>(b, P, dissip_on, (int)(t - row));
+  else if (t < 3 * row) body_prep_dir<T, FAST, S, 2>(b, P, dissip_on, (int)(t - 2 * row));
+}
+template <typename T, bool FAST, bool S>
+__device__ __forceinline__ void body_face_rows(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd,
+                                               long long t) {
+  const long long row = split_row(b, 1);
+  if (t < row) body_face_split<T, FAST, S, 0>(b, P, dissip_on, cd, (int)t);
+  else if (t < 2 * row) body_face_split<T, FAST, S, 1>(b, P, dissip_on, cd, (int)(t - row));
+  else if (t < 3 * row) body_face_split<T, FAST, S, 2>(b, P, dissip_on, cd, (int)(t - 2 * row));
 }
 
 // --------------------------------------------------------------- stage: cut-cell record terms
@@ -1030,13 +1135,12 @@ __device__ __forceinline__ T unsteady_lam(const DevBlock<T>& b, const PhysParams
 // is the central difference of the cell fluxes, efs(q) - efs(q+1) =
 // 0.5*(F(q-1) - F(q+1)) in each direction, so no convective face pass runs;
 // a record's dense face pair takes the same difference.
-template <typename T, bool FAST = false>
+template <typename T, bool FAST = false, bool S = true>
 __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysParams& P, const StageArgs& A,
                                              unsigned* err, long long t) {
   const int nxl = b.nx, nyl = b.ny;
-  int i = 2 + (int)(t % nxl);
-  int j = 2 + (int)((t / nxl) % nyl);
-  int k = 2 + (int)(t / ((long long)nxl * nyl));
+  int i, j, k;
+  cell_of(t, nxl, nyl, 2, i, j, k);
   const long long N = b.N;
   const long long c = cidx(b.Pi, b.Pj, i, j, k);
   const long long sj = b.Pi, sk = (long long)b.Pi * b.Pj;
@@ -1071,7 +1175,7 @@ __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysPar
     const T* Dz = b.dfs + 10 * N;
     T vis[5];
 #pragma unroll
-    for (int v = 0; v < 5; v++) vis[v] = A.scale_fw ? smul(b.fw[v * N + c], fac) : T(0);
+    for (int v = 0; v < 5; v++) vis[v] = A.scale_fw ? pmul<S>(b.fw[v * N + c], fac) : T(0);
     if (P.eqn_ns) {  // viscous faces, then the viscous wall faces in record order
       const T* Vx = b.vfs;
       const T* Vy = b.vfs + 5 * N;
@@ -1124,7 +1228,7 @@ __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysPar
     }
   } else {
 #pragma unroll
-    for (int v = 0; v < 5; v++) fwv[v] = A.scale_fw ? smul(b.fw[v * N + c], fac) : T(0);
+    for (int v = 0; v < 5; v++) fwv[v] = A.scale_fw ? pmul<S>(b.fw[v * N + c], fac) : T(0);
   }
   if (tg >= 0) {
     // cut-cell wall faces, this cell's records in record order: efluxb on dw
@@ -1223,9 +1327,9 @@ __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysPar
   }
   // time-step scaling, euler.f90:364-372: de = fn*vdtim/cellvolume
   T vd = A.vt ? (T)(*b.dtim) : b.vdtim[c];
-  T de = FAST ? ((T)A.fn * vd) * rcp_vol(b) : smdiv(smul((T)A.fn, vd), (T)b.vol, rcp_vol(b));
+  T de = FAST ? ((T)A.fn * vd) * rcp_vol(b) : pmdiv<S>(pmul<S>((T)A.fn, vd), (T)b.vol, rcp_vol(b));
 #pragma unroll
-  for (int v = 0; v < 5; v++) dwv[v] = smul(de, dwv[v]);
+  for (int v = 0; v < 5; v++) dwv[v] = pmul<S>(de, dwv[v]);
   if (A.irs) {
 #pragma unroll
     for (int v = 0; v < 5; v++) b.dw[v * N + c] = dwv[v];
@@ -1246,7 +1350,7 @@ __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysPar
     b.w[v * N + c] = wv[v];
     b.dw[v * N + c] = dwv[v];
   }
-  b.p[c] = depvars((T)P.gamma, wv);
+  b.p[c] = depvars<S>((T)P.gamma, wv);
 }
 
 // --------------------------------------------------------------- implicit residual smoothing
@@ -1260,6 +1364,11 @@ __device__ __forceinline__ long long irs_lines(const DevBlock<T>& b) {
   return D == 0 ? (long long)b.ny * b.nz : (D == 1 ? (long long)b.nx * b.nz : (long long)b.nx * b.ny);
 }
 
+// the variable of (line, variable) item t: t / lines, which is 0..4
+__device__ __forceinline__ int line_var(long long t, long long lines) {
+  return (t >= lines) + (t >= 2 * lines) + (t >= 3 * lines) + (t >= 4 * lines);
+}
+
 // SC: the products of the forward and backward steps on the integer pipes.
 // That lengthens the serial chain of each line, so it pays only where many
 // lines run at once and the sweep is bound by the FP64 rate; with few lines
@@ -1268,22 +1377,22 @@ __device__ __forceinline__ long long irs_lines(const DevBlock<T>& b) {
 template <typename T, typename TC, int D, bool SC = false>
 __device__ __forceinline__ void body_irs(const DevBlock<T>& b, const IrsTables& tb, TC bb, long long t) {
   const long long lines = irs_lines<T, D>(b);
-  const int v = (int)(t / lines);
+  const int v = line_var(t, lines);
   const long long ln = t - (long long)v * lines;
   long long c0, st;
   int l;
   if (D == 0) {
-    int j = 2 + (int)(ln % b.ny), k = 2 + (int)(ln / b.ny);
+    int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
     c0 = cidx(b.Pi, b.Pj, 0, j, k);
     st = 1;
     l = b.il;
   } else if (D == 1) {
-    int i = 2 + (int)(ln % b.nx), k = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), k = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, 0, k);
     st = b.Pi;
     l = b.jl;
   } else {
-    int i = 2 + (int)(ln % b.nx), j = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), j = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, j, 0);
     st = (long long)b.Pi * b.Pj;
     l = b.kl;
@@ -1363,22 +1472,22 @@ __device__ __forceinline__ void body_irs_mixed(const DevBlock<double>& b, const 
   constexpr bool fill = !std::is_same<TS, float>::value;  // the i sweep: every cell into the copy
   constexpr bool back = !std::is_same<TO, float>::value;  // the k sweep: results back to dw
   const long long lines = irs_lines<double, D>(b);
-  const int v = (int)(t / lines);
+  const int v = line_var(t, lines);
   const long long ln = t - (long long)v * lines;
   long long c0, st;
   int l;
   if (D == 0) {
-    int j = 2 + (int)(ln % b.ny), k = 2 + (int)(ln / b.ny);
+    int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
     c0 = cidx(b.Pi, b.Pj, 0, j, k);
     st = 1;
     l = b.il;
   } else if (D == 1) {
-    int i = 2 + (int)(ln % b.nx), k = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), k = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, 0, k);
     st = b.Pi;
     l = b.jl;
   } else {
-    int i = 2 + (int)(ln % b.nx), j = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), j = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, j, 0);
     st = (long long)b.Pi * b.Pj;
     l = b.kl;
@@ -1466,9 +1575,9 @@ __global__ void __launch_bounds__(256) k_irs_scan_i(DevBlock<T> b, IrsTables tb,
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= 5 * lines) return;  // uniform over the warp
-  const int v = (int)(wid / lines);
+  const int v = line_var(wid, lines);
   const long long ln = wid - (long long)v * lines;
-  const int j = 2 + (int)(ln % b.ny), k = 2 + (int)(ln / b.ny);
+  const int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
   const long long c0 = cidx(b.Pi, b.Pj, 0, j, k);
   const int l = b.il;
   const T* src = b.dw + (long long)v * b.N + c0;  // read whole into registers before any write
@@ -1594,13 +1703,13 @@ __device__ __forceinline__ void body_irs_smem(const DevBlock<T>& b, const IrsTab
   auto cell = [&](int r, int q) -> long long {
     long long ln = l0 + r;
     if (D == 0) {
-      int j = 2 + (int)(ln % b.ny), k = 2 + (int)(ln / b.ny);
+      int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
       return cidx(b.Pi, b.Pj, 2 + q, j, k);
     } else if (D == 1) {
-      int i = 2 + (int)(ln % b.nx), k = 2 + (int)(ln / b.nx);
+      int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), k = 2 + (int)((unsigned)ln / (unsigned)b.nx);
       return cidx(b.Pi, b.Pj, i, 2 + q, k);
     } else {
-      int i = 2 + (int)(ln % b.nx), j = 2 + (int)(ln / b.nx);
+      int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), j = 2 + (int)((unsigned)ln / (unsigned)b.nx);
       return cidx(b.Pi, b.Pj, i, j, 2 + q);
     }
   };
@@ -1682,17 +1791,17 @@ size_t irs_smem_bytes(int len) {
 template <typename T, int D>
 __device__ __forceinline__ void line_of(const DevBlock<T>& b, long long ln, long long& c0, long long& st, int& l) {
   if (D == 0) {
-    int j = 2 + (int)(ln % b.ny), k = 2 + (int)(ln / b.ny);
+    int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
     c0 = cidx(b.Pi, b.Pj, 0, j, k);
     st = 1;
     l = b.il;
   } else if (D == 1) {
-    int i = 2 + (int)(ln % b.nx), k = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), k = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, 0, k);
     st = b.Pi;
     l = b.jl;
   } else {
-    int i = 2 + (int)(ln % b.nx), j = 2 + (int)(ln / b.nx);
+    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), j = 2 + (int)((unsigned)ln / (unsigned)b.nx);
     c0 = cidx(b.Pi, b.Pj, i, j, 0);
     st = (long long)b.Pi * b.Pj;
     l = b.kl;
@@ -1776,12 +1885,11 @@ __global__ void k_psmoo_line(DevBlock<T> b) {
   if (t < irs_lines<T, D>(b)) body_psmoo_line<T, TC, D>(b, t);
 }
 
-template <typename T>
+template <typename T, bool S = true>
 __device__ __forceinline__ void body_update(const DevBlock<T>& b, const PhysParams& P, const StageArgs& A,
                                             long long t) {
-  int i = 2 + (int)(t % b.nx);
-  int j = 2 + (int)((t / b.nx) % b.ny);
-  int k = 2 + (int)(t / ((long long)b.nx * b.ny));
+  int i, j, k;
+  cell_of(t, b.nx, b.ny, 2, i, j, k);
   const long long N = b.N;
   const long long c = cidx(b.Pi, b.Pj, i, j, k);
   T wv[5];
@@ -1795,7 +1903,7 @@ __device__ __forceinline__ void body_update(const DevBlock<T>& b, const PhysPara
   }
 #pragma unroll
   for (int v = 0; v < 5; v++) b.w[v * N + c] = wv[v];
-  b.p[c] = depvars((T)P.gamma, wv);
+  b.p[c] = depvars<S>((T)P.gamma, wv);
 }
 
 // --------------------------------------------------------------- bc_cutcell (bc_cutcell.f90:40-268)
@@ -1860,14 +1968,6 @@ __device__ __forceinline__ double pow_gamma(const PhysParams& P, double x, doubl
   return pow(x, gamma);
 }
 __device__ __forceinline__ float pow_gamma(const PhysParams&, float x, float gamma) { return pow(x, gamma); }
-
-// depvars with plain products: the same bits as depvars(), and the shorter
-// dependent chain (32 cycles a product against about 100 for smul) where few
-// cells are worked on and the FP64 pipe is idle
-template <typename T> __device__ __forceinline__ T depvars_plain(T gamma, const T* w) {
-  const T qq = T(0.5) * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) / w[0];
-  return (gamma - T(1)) * fdimT(w[4], qq);
-}
 
 template <typename T> struct CellState {
   T w[5];
@@ -2229,11 +2329,11 @@ __device__ __forceinline__ void body_bc_corner(const DevBlock<T>& b, const PhysP
       o.w[v] = mdiv((e.w[v] + bq + cq) * T(2), T(3), T(1) / T(3)) - d;
     }
     if (asis) {
-      e.p = depvars_plain(gamma, e.w);
+      e.p = depvars<false>(gamma, e.w);
       store_cell(b, cidx(b.Pi, b.Pj, ii, j, k), e);
     }
   }
-  o.p = depvars_plain(gamma, o.w);
+  o.p = depvars<false>(gamma, o.w);
   store_cell(b, cidx(b.Pi, b.Pj, i, j, k), o);
 }
 
@@ -2275,20 +2375,8 @@ __device__ void body_rtrms_partial(const DevBlock<T>& b, double cfl, int vt, dou
   const long long lo = (long long)part * per, hi = min(tot, lo + per);
   double acc = 0.0;
   for (long long t = lo + threadIdx.x; t < hi; t += blockDim.x) {
-    // 32-bit index arithmetic while the block's cells fit (the same cells)
     int i, j, k;
-    if (tot < (1ll << 31)) {
-      const int t32 = (int)t, nxy = b.nx * b.ny;
-      k = t32 / nxy;
-      const int r = t32 - k * nxy;
-      j = r / b.nx;
-      i = r - j * b.nx;
-      i += 2, j += 2, k += 2;
-    } else {
-      i = 2 + (int)(t % b.nx);
-      j = 2 + (int)((t / b.nx) % b.ny);
-      k = 2 + (int)(t / ((long long)b.nx * b.ny));
-    }
+    cell_of(t, b.nx, b.ny, 2, i, j, k);
     long long c = cidx(b.Pi, b.Pj, i, j, k);
     double de = smul(cfl, (double)(vt ? *b.dtim : b.vdtim[c]));
     double rt = 0.0;
@@ -2356,9 +2444,8 @@ __global__ void k_copy5(const T* __restrict__ src, T* __restrict__ dst, long lon
 template <typename T>
 __device__ __forceinline__ void body_save_wn(const DevBlock<T>& b, long long c) {
   const long long N = b.N;
-  int i = (int)(c % b.Pi);
-  int j = (int)((c / b.Pi) % b.Pj);
-  int k = (int)(c / ((long long)b.Pi * b.Pj));
+  int i, j, k;
+  cell_of(c, b.Pi, b.Pj, 0, i, j, k);
   bool phys = i >= 2 && i <= b.il && j >= 2 && j <= b.jl && k >= 2 && k <= b.kl;
   for (int v = 0; v < 5; v++) {
     if (phys) b.wn[v * N + c] = b.w[v * N + c];
@@ -2377,9 +2464,8 @@ __global__ void k_save_wn(DevBlock<T> b) {
 template <typename T>
 __device__ __forceinline__ void body_copy_wn(const DevBlock<T>& b, long long c) {
   if (c >= b.N) return;
-  int i = (int)(c % b.Pi);
-  int j = (int)((c / b.Pi) % b.Pj);
-  int k = (int)(c / ((long long)b.Pi * b.Pj));
+  int i, j, k;
+  cell_of(c, b.Pi, b.Pj, 0, i, j, k);
   if (!(i >= 2 && i <= b.il && j >= 2 && j <= b.jl && k >= 2 && k <= b.kl)) return;
   for (int v = 0; v < 5; v++) b.wn[v * b.N + c] = b.w[v * b.N + c];
 }
@@ -2428,7 +2514,9 @@ __device__ __forceinline__ void body_collc(const DevBlock<TC>& c, const DevBlock
                                            uint8_t* marker, long long t) {
   const int n0 = f.nx / X.r[0], n1 = f.ny / X.r[1], n2 = f.nz / X.r[2];
   if (t >= (long long)n0 * n1 * n2) return;
-  int ic[3] = {X.o[0] + 2 + (int)(t % n0), X.o[1] + 2 + (int)((t / n0) % n1), X.o[2] + 2 + (int)(t / ((long long)n0 * n1))};
+  int ic[3];
+  cell_of(t, n0, n1, 2, ic[0], ic[1], ic[2]);
+  for (int d = 0; d < 3; d++) ic[d] += X.o[d];
   if (ic[0] < 2 || ic[0] > c.il || ic[1] < 2 || ic[1] > c.jl || ic[2] < 2 || ic[2] > c.kl) return;
   const int lf[3] = {f.il, f.jl, f.kl};
   if constexpr (std::is_same<TC, float>::value && std::is_same<TF, double>::value) {
@@ -2544,7 +2632,8 @@ template <typename TF, typename TC>
 __device__ __forceinline__ void body_addw(const DevBlock<TF>& f, const DevBlock<TC>& c, const Xfer& X, int fmg,
                                           const double* dc, long long t) {
   if (t >= (long long)f.nx * f.ny * f.nz) return;
-  int i = 2 + (int)(t % f.nx), j = 2 + (int)((t / f.nx) % f.ny), k = 2 + (int)(t / ((long long)f.nx * f.ny));
+  int i, j, k;
+  cell_of(t, f.nx, f.ny, 2, i, j, k);
   if constexpr (std::is_same<TF, double>::value && std::is_same<TC, float>::value) {
     // the mixed form's finest level under an FP32 coarse level: the coarse
     // correction is FP32, so it is interpolated in FP32 (the same stencil
@@ -2638,7 +2727,8 @@ template <typename TF, typename TC>
 __device__ __forceinline__ void body_embed(const DevBlock<TF>& f, const DevBlock<TC>& c, const Xfer& X, double gamma,
                                            long long t) {
   if (t >= f.N) return;
-  int i = (int)(t % f.Pi), j = (int)((t / f.Pi) % f.Pj), k = (int)(t / ((long long)f.Pi * f.Pj));
+  int i, j, k;
+  cell_of(t, f.Pi, f.Pj, 0, i, j, k);
   if (i >= 2 && i <= f.il && j >= 2 && j <= f.jl && k >= 2 && k <= f.kl) return;
   int sh[3];
   double fac[8];
@@ -2674,7 +2764,8 @@ __global__ void k_solut(DevBlock<T> b, double gamma, double p0, double rm, doubl
   const long long ncell = (long long)b.nx * b.ny * b.nz;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncell) return;
-  const int i = 2 + (int)(t % b.nx), j = 2 + (int)((t / b.nx) % b.ny), k = 2 + (int)(t / ((long long)b.nx * b.ny));
+  int i, j, k;
+  cell_of(t, b.nx, b.ny, 2, i, j, k);
   const long long N = b.N, c = cidx(b.Pi, b.Pj, i, j, k);
   const double rr = (double)b.w[c];
   const double uu = (double)b.w[N + c] / rr;
@@ -2755,10 +2846,10 @@ __global__ void k_forces(DevBlock<T> b, double ox, double oy, double oz, double 
 }
 
 // =============================================================== one-launch-per-phase kernels
-template <typename T, bool SLOPES, bool FAST = false>
-__global__ void __launch_bounds__(256, SLOPES ? 3 : 6) k_prep(DevBlock<T> b, PhysParams P, int dissip_on) {
+template <typename T, bool SLOPES, bool FAST, bool S>
+__global__ void __launch_bounds__(256, SLOPES ? 3 : (S ? 6 : 4)) k_prep(DevBlock<T> b, PhysParams P, int dissip_on) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)b.ie * b.je * b.ke) body_prep<T, SLOPES, FAST>(b, P, dissip_on, t);
+  if (t < (long long)b.ie * b.je * b.ke) body_prep<T, SLOPES, FAST, S>(b, P, dissip_on, t);
 }
 // the velocities of every cell, ghosts included, into F[0..2] for the MUSCL
 // Roe form (one reciprocal of the density and mdiv: the IEEE quotients)
@@ -2777,16 +2868,25 @@ __global__ void __launch_bounds__(256, 4)
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL>(b, P, dissip_on, cd, t);
 }
-template <typename T>
-__global__ void __launch_bounds__(256, 6) k_face_jst(DevBlock<T> b, PhysParams P, int dissip_on, T cd) {
+template <typename T, bool S>
+__global__ void __launch_bounds__(256, S ? 6 : 4) k_face_jst(DevBlock<T> b, PhysParams P, int dissip_on, T cd) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_JST>(b, P, dissip_on, cd, t);
+  if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_JST, S>(b, P, dissip_on, cd, t);
 }
-// the contracted form's dissipation faces (no convective face fluxes)
-template <typename T>
-__global__ void __launch_bounds__(256, 4) k_face_diss(DevBlock<T> b, PhysParams P, T cd) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face_diss<T>(b, P, cd, t);
+// the prep and face passes of a small level, one direction per grid row
+template <typename T, bool FAST, bool S>
+__global__ void __launch_bounds__(256) k_prep_split(DevBlock<T> b, PhysParams P, int dissip_on) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) body_prep_dir<T, FAST, S, 0>(b, P, dissip_on, t);
+  else if (blockIdx.y == 1) body_prep_dir<T, FAST, S, 1>(b, P, dissip_on, t);
+  else body_prep_dir<T, FAST, S, 2>(b, P, dissip_on, t);
+}
+template <typename T, bool FAST, bool S>
+__global__ void __launch_bounds__(256) k_face_split(DevBlock<T> b, PhysParams P, int dissip_on, T cd) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) body_face_split<T, FAST, S, 0>(b, P, dissip_on, cd, t);
+  else if (blockIdx.y == 1) body_face_split<T, FAST, S, 1>(b, P, dissip_on, cd, t);
+  else body_face_split<T, FAST, S, 2>(b, P, dissip_on, cd, t);
 }
 // the Roe faces (MUSCL states, upwind flux, and the viscous flux with NS)
 template <typename T>
@@ -2802,7 +2902,8 @@ template <typename T>
 __device__ __forceinline__ void body_face_conv(const DevBlock<T>& b, long long t) {
   const int ex = b.ie - 1, ey = b.je - 1;
   if (t >= (long long)ex * ey * (b.ke - 1)) return;
-  const int i = 2 + (int)(t % ex), j = 2 + (int)((t / ex) % ey), k = 2 + (int)(t / ((long long)ex * ey));
+  int i, j, k;
+  cell_of(t, ex, ey, 2, i, j, k);
   const long long N = b.N, c = cidx(b.Pi, b.Pj, i, j, k);
   const bool on[3] = {j <= b.jl && k <= b.kl, i <= b.il && k <= b.kl, i <= b.il && j <= b.jl};
   const long long sts[3] = {1, (long long)b.Pi, (long long)b.Pi * b.Pj};
@@ -2819,20 +2920,20 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_face_conv(DevBlock<T> b) {
   body_face_conv(b, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
-template <typename T, bool FAST = false>
+template <typename T, bool FAST, bool S>
 __global__ void k_combine(DevBlock<T> b, PhysParams P, StageArgs A, unsigned* err) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST>(b, P, A, err, t);
+  if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST, S>(b, P, A, err, t);
 }
 template <typename T, typename TC, int D, bool SC = false>
 __global__ void k_irs(DevBlock<T> b, IrsTables tb, TC bb) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 5 * irs_lines<T, D>(b)) body_irs<T, TC, D, SC>(b, tb, bb, t);
 }
-template <typename T>
+template <typename T, bool S>
 __global__ void k_update(DevBlock<T> b, PhysParams P, StageArgs A) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)b.nx * b.ny * b.nz) body_update(b, P, A, t);
+  if (t < (long long)b.nx * b.ny * b.nz) body_update<T, S>(b, P, A, t);
 }
 template <typename T>
 __global__ void k_cutcell(DevBlock<T> b, PhysParams P, unsigned* err) {
@@ -2888,7 +2989,7 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
     for (long long base = (long long)blockIdx.x * blockDim.x; base < ncell; base += gs) {
       long long t = base + threadIdx.x;
       unsigned long long mine = ~0ull;
-      if (t < ncell) mine = body_timestep<T, TA>(b, P, E.err, t);
+      if (t < ncell) mine = body_timestep<T, TA, false>(b, P, E.err, t);
       block_min_to(mine, b.dtim);
     }
     g.sync();
@@ -2902,21 +3003,22 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
   for (int m = 1; m <= E.mstage; m++) {
     const StageArgs& A = E.st[m - 1];
     if (A.fast) {
-      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, true>(b, P, A.dissip_on, t);
+      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, true, false>(b, P, A.dissip_on, t);
       g.sync();
       if (A.dissip_on)
-        for (long long t = gt; t < nface; t += gs) body_face_diss(b, P, (T)A.cd, t);
+        for (long long t = gt; t < 3 * split_row(b, 1); t += gs)
+          body_face_rows<T, true, false>(b, P, 1, (T)A.cd, t);
     } else {
-      for (long long t = gt; t < nprep; t += gs) body_prep(b, P, A.dissip_on, t);
+      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, false, false>(b, P, A.dissip_on, t);
       g.sync();
-      for (long long t = gt; t < nface; t += gs) body_face(b, P, A.dissip_on, (T)A.cd, t);
+      for (long long t = gt; t < nface; t += gs) body_face<T, FACE_ANY, false>(b, P, A.dissip_on, (T)A.cd, t);
     }
     for (long long t = gt; t < b.nmir; t += gs) rec_wall_terms(b, P, A.dissip_on, (T)A.cd, E.err, (int)t);
     g.sync();
     if (A.fast)
-      for (long long t = gt; t < ncell; t += gs) body_combine<T, true>(b, P, A, E.err, t);
+      for (long long t = gt; t < ncell; t += gs) body_combine<T, true, false>(b, P, A, E.err, t);
     else
-      for (long long t = gt; t < ncell; t += gs) body_combine<T>(b, P, A, E.err, t);
+      for (long long t = gt; t < ncell; t += gs) body_combine<T, false, false>(b, P, A, E.err, t);
     g.sync();
     if (E.lres) return;
     if (A.irs && P.irs_kind == 1) {
@@ -2936,7 +3038,7 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
       g.sync();
     }
     if (A.irs) {
-      for (long long t = gt; t < ncell; t += gs) body_update(b, P, A, t);
+      for (long long t = gt; t < ncell; t += gs) body_update<T, false>(b, P, A, t);
       g.sync();
     }
     for (long long t = gt; t < b.nmir; t += gs) body_cutcell(b, P, E.err, (int)t);
@@ -3005,11 +3107,11 @@ template <typename T> struct FDtimReset {
     if (t == 0) *M.B[q].dtim = 10.0;
   }
 };
-template <typename T, typename TC> struct FTimestep {
+template <typename T, typename TC, bool S> struct FTimestep {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
     unsigned long long mine = ~0ull;
-    if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC>(b, M.P[q], M.err[q], t);
+    if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC, S>(b, M.P[q], M.err[q], t);
     block_min_to(mine, b.dtim);
   }
 };
@@ -3024,29 +3126,35 @@ template <typename T> struct FSaveWn {
     if (t < M.B[q].N) body_save_wn(M.B[q], t);
   }
 };
-template <typename T, bool FAST> struct FPrep {
+template <typename T, bool FAST, bool S> struct FPrep {
   int dissip_on;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, false, FAST>(b, M.P[q], dissip_on, t);
+    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, false, FAST, S>(b, M.P[q], dissip_on, t);
   }
 };
-template <typename T> struct FFace {
+template <typename T, bool S> struct FFace {
   int dissip_on;
   T cd;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL>(b, M.P[q], dissip_on, cd, t);
+    if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL, S>(b, M.P[q], dissip_on, cd, t);
   }
 };
 template <typename T> struct FFaceConv {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const { body_face_conv(M.B[q], t); }
 };
-template <typename T> struct FFaceDiss {
+template <typename T, bool FAST, bool S> struct FPrepRows {
+  int dissip_on;
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
+    body_prep_rows<T, FAST, S>(M.B[q], M.P[q], dissip_on, t);
+  }
+};
+template <typename T, bool FAST, bool S> struct FFaceRows {
+  int dissip_on;
   T cd;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
-    if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face_diss<T>(b, M.P[q], cd, t);
+    body_face_rows<T, FAST, S>(M.B[q], M.P[q], dissip_on, cd, t);
   }
 };
 template <typename T> struct FRec {
@@ -3056,11 +3164,11 @@ template <typename T> struct FRec {
     if (t < M.B[q].nmir) rec_wall_terms(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
   }
 };
-template <typename T, bool FAST> struct FCombine {
+template <typename T, bool FAST, bool S> struct FCombine {
   StageArgs A;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST>(b, M.P[q], A, M.err[q], t);
+    if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST, S>(b, M.P[q], A, M.err[q], t);
   }
 };
 template <typename T, typename TC, int D> struct FIrs {
@@ -3080,11 +3188,11 @@ template <typename TS, typename TO, int D> struct FIrsMixed {
     body_irs_mixed<TS, TO, D>(b, M.tab[3 * q + D], (float)(-M.P[q].smoo), src, cp, out, t);
   }
 };
-template <typename T> struct FUpdate {
+template <typename T, bool S> struct FUpdate {
   StageArgs A;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.nx * b.ny * b.nz) body_update(b, M.P[q], A, t);
+    if (t < (long long)b.nx * b.ny * b.nz) body_update<T, S>(b, M.P[q], A, t);
   }
 };
 template <typename T> struct FCutcell {
@@ -3182,6 +3290,34 @@ inline int tpb_for(long long n) {
 }
 #define LAUNCH_N(n) nblk((n), tpb_for(n)), tpb_for(n)
 
+// FP64 blocks of up to this many cells run plain FP64 operations instead of
+// the integer-pipe forms (pmul).  Measured, plain against integer: a W-cycle's
+// 24^3 update 269 against 281 us, a 64x64x2 one 402 against 421; a 48^3 level's
+// cycle 1.18 against 1.09 ms, a 192^3 one 50 against 40.
+constexpr long long kPlainCells = 32768;
+template <typename T> bool on_int_pipes(const DevBlock<T>& b) {
+  return (long long)b.nx * b.ny * b.nz > kPlainCells;
+}
+// f(std::true_type) with the integer-pipe forms, f(std::false_type) without; FP32 has one form
+template <typename T, typename F> void with_form(const DevBlock<T>& b, F&& f) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (!on_int_pipes(b)) return f(std::false_type{});
+  }
+  f(std::true_type{});
+}
+
+// Passes with one thread per cell and direction (body_prep_dir,
+// body_face_split).  A level that leaves schedulers without a warp gains from
+// the shorter threads; a large one pays for the values read and formed three
+// times.  Measured, split against whole, us: FP64 24^3 prep 9.8 against 11.8 and
+// face 11 against 18; 48^3 21 against 27 and 22 against 27; 96^3 prep 112 against
+// 120 but face 134 against 124; 192^3 face 962 against 897.  The contracted
+// dissipation faces share nothing between the directions, and split they keep
+// twice the warps resident: 414 against 563 us a launch at 192^3.
+inline bool split_scheme(const PhysParams& P) { return P.distype == 0 && !P.eqn_ns && !P.matrix; }
+inline bool split_prep(bool fast, long long cells) { return cells <= (fast ? 300000 : 1000000); }
+inline bool split_face(bool fast, long long cells) { return fast || cells <= 300000; }
+
 template <typename T>
 void launch_solut(const DevBlock<T>& b, const PhysParams& P, double rm, double p_tot, int ns, double* out,
                   cudaStream_t s) {
@@ -3194,33 +3330,56 @@ template <typename T>
 void launch_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s, bool aux32) {
   long long n = (long long)b.nx * b.ny * b.nz;
   k_dtim_reset<<<1, 32, 0, s>>>(b.dtim);
-  if (aux32)
-    k_timestep<T, float><<<LAUNCH_N(n), 0, s>>>(b, P, err);
-  else
-    k_timestep<T, T><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+  with_form(b, [&](auto S) {
+    if (aux32)
+      k_timestep<T, float, true><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+    else
+      k_timestep<T, T, S.value><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+  });
 }
 
 template <typename T>
 void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, const StageArgs& A, unsigned* err,
                        cudaStream_t s) {
-  if (part == 0) {
+  const long long cells = (long long)b.nx * b.ny * b.nz;
+  // the largest direction's items of a split pass (e = 2: prep, 1: faces), a row of the grid each
+  auto rows = [&](int e) {
+    const long long n = std::max({(long long)(b.nx + e) * b.ny * b.nz, (long long)b.nx * (b.ny + e) * b.nz,
+                                  (long long)b.nx * b.ny * (b.nz + e)});
+    return std::make_pair(dim3(nblk(n, tpb_for(3 * n)), 3), tpb_for(3 * n));
+  };
+  if (part == 0 && split_scheme(P) && split_prep(A.fast, cells)) {
+    const auto g = rows(2);
+    with_form(b, [&](auto S) {
+      if (A.fast)
+        k_prep_split<T, true, S.value><<<g.first, g.second, 0, s>>>(b, P, A.dissip_on);
+      else
+        k_prep_split<T, false, S.value><<<g.first, g.second, 0, s>>>(b, P, A.dissip_on);
+    });
+  } else if (part == 1 && split_scheme(P) && split_face(A.fast, cells)) {
+    const auto g = rows(1);
+    with_form(b, [&](auto S) {
+      if (!A.fast)
+        k_face_split<T, false, S.value><<<g.first, g.second, 0, s>>>(b, P, A.dissip_on, (T)A.cd);
+      else if (A.dissip_on)
+        k_face_split<T, true, S.value><<<g.first, g.second, 0, s>>>(b, P, 1, (T)A.cd);
+    });
+  } else if (part == 0) {
     long long n1 = (long long)b.ie * b.je * b.ke;
     if (A.fast) {
-      k_prep<T, false, true><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+      with_form(b, [&](auto S) { k_prep<T, false, true, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on); });
     } else if (P.distype == 2) {
       k_prim<T><<<LAUNCH_N(b.N), 0, s>>>(b);
-      k_prep<T, true><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+      k_prep<T, true, false, true><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
     } else {
-      k_prep<T, false><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+      with_form(b, [&](auto S) { k_prep<T, false, false, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on); });
     }
   } else if (part == 1) {
     long long n2 = (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1);
-    if (A.fast) {
-      if (A.dissip_on) k_face_diss<T><<<LAUNCH_N(n2), 0, s>>>(b, P, (T)A.cd);
-    } else if (!A.dissip_on && P.distype == 0)
+    if (!A.dissip_on && P.distype == 0)
       k_face_conv<T><<<LAUNCH_N(n2), 0, s>>>(b);
     else if (P.distype == 0 && !P.eqn_ns && !P.matrix)
-      k_face_jst<T><<<LAUNCH_N(n2), 0, s>>>(b, P, A.dissip_on, (T)A.cd);
+      with_form(b, [&](auto S) { k_face_jst<T, S.value><<<LAUNCH_N(n2), 0, s>>>(b, P, A.dissip_on, (T)A.cd); });
     else if (P.distype == 0)
       k_face<T><<<LAUNCH_N(n2), 0, s>>>(b, P, A.dissip_on, (T)A.cd);
     else
@@ -3229,10 +3388,12 @@ void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, cons
     if (b.nmir > 0) k_rec_wall<T><<<LAUNCH_N(b.nmir), 0, s>>>(b, P, A.dissip_on, (T)A.cd, err);
   } else if (part == 3) {
     long long n3 = (long long)b.nx * b.ny * b.nz;
-    if (A.fast)
-      k_combine<T, true><<<LAUNCH_N(n3), 0, s>>>(b, P, A, err);
-    else
-      k_combine<T><<<LAUNCH_N(n3), 0, s>>>(b, P, A, err);
+    with_form(b, [&](auto S) {
+      if (A.fast)
+        k_combine<T, true, S.value><<<LAUNCH_N(n3), 0, s>>>(b, P, A, err);
+      else
+        k_combine<T, false, S.value><<<LAUNCH_N(n3), 0, s>>>(b, P, A, err);
+    });
   }
 }
 
@@ -3309,7 +3470,7 @@ void launch_irs_part_t(int part, const DevBlock<T>& b, const PhysParams& P, cons
     if (part == 1) k_psmoo_line<T, TC, 1><<<LAUNCH_N(irs_lines_h(b, 1)), 0, s>>>(b);
     if (part == 2) {
       k_psmoo_line<T, TC, 2><<<LAUNCH_N(irs_lines_h(b, 2)), 0, s>>>(b);
-      k_update<T><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au);
+      with_form(b, [&](auto S) { k_update<T, S.value><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au); });
     }
     return;
   }
@@ -3339,7 +3500,7 @@ void launch_irs_part_t(int part, const DevBlock<T>& b, const PhysParams& P, cons
       k_irs_mixed<float, float, 1><<<LAUNCH_N(5 * irs_lines_h(b, 1)), 0, s>>>(b, tab[1], bb, cp, cp, cp);
     if (part == 2) {
       k_irs_mixed<float, double, 2><<<LAUNCH_N(5 * irs_lines_h(b, 2)), 0, s>>>(b, tab[2], bb, cp, cp, b.dw);
-      k_update<T><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au);
+      with_form(b, [&](auto S) { k_update<T, S.value><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au); });
     }
     return;
   }
@@ -3347,7 +3508,7 @@ void launch_irs_part_t(int part, const DevBlock<T>& b, const PhysParams& P, cons
   if (part == 1) launch_irs_dir<T, TC, 1>(b, tab[1], bb, s, variant ? variant[1] : 0);
   if (part == 2) {
     launch_irs_dir<T, TC, 2>(b, tab[2], bb, s, variant ? variant[2] : 0);
-    k_update<T><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au);
+    with_form(b, [&](auto S) { k_update<T, S.value><<<LAUNCH_N(ncell), 0, s>>>(b, P, Au); });
   }
 }
 
@@ -3383,6 +3544,15 @@ void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s, boo
 template <typename T>
 long long bc_items(const DevBlock<T>& b, int part) {
   return bc_items_t(b, part);
+}
+
+template <typename T>
+long long split_items(const DevBlock<T>& b, int e) {
+  return split_items_t(b, e);
+}
+void split_passes(const PhysParams& P, bool fast, long long cells, bool* prep, bool* face) {
+  *prep = split_scheme(P) && split_prep(fast, cells);
+  *face = split_scheme(P) && split_face(fast, cells);
 }
 
 template <typename T>
@@ -3586,36 +3756,43 @@ static void multi_bcond(const MultiLevel& L, MultiArgs<T>& M, cudaStream_t s, bo
 
 // timestep (optionally) and euler.f90:1-462 on one block of every case: the
 // phases of enqueue_euler's per-phase path (line sweeps in global memory)
-template <typename T>
+template <typename T, bool S>
 static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, bool with_timestep, bool lfir,
                           bool rt, cudaStream_t s) {
   MultiArgs<T> M = multi_args<T>(L);
   if (with_timestep) {
     go_multi(L, M, MK_ONE, FDtimReset<T>{}, s);
     if (L.aux32)
-      go_multi(L, M, MK_PHYS, FTimestep<T, float>{}, s);
+      go_multi(L, M, MK_PHYS, FTimestep<T, float, true>{}, s);
     else
-      go_multi(L, M, MK_PHYS, FTimestep<T, T>{}, s);
+      go_multi(L, M, MK_PHYS, FTimestep<T, T, S>{}, s);
   }
   if (lfir) go_multi(L, M, MK_N5, FCopyWs<T>{}, s);
   go_multi(L, M, MK_N, FSaveWn<T>{}, s);
   for (int m = 1; m <= mstage; m++) {
     const StageArgs& a = A[m - 1];
+    if (L.prep_rows && L.fast)
+      go_multi(L, M, MK_PREP3, FPrepRows<T, true, S>{a.dissip_on}, s);
+    else if (L.prep_rows)
+      go_multi(L, M, MK_PREP3, FPrepRows<T, false, S>{a.dissip_on}, s);
+    else if (L.fast)
+      go_multi(L, M, MK_PREP, FPrep<T, true, S>{a.dissip_on}, s);
+    else
+      go_multi(L, M, MK_PREP, FPrep<T, false, S>{a.dissip_on}, s);
     if (L.fast) {
-      go_multi(L, M, MK_PREP, FPrep<T, true>{a.dissip_on}, s);
-      if (a.dissip_on) go_multi(L, M, MK_FACE, FFaceDiss<T>{(T)a.cd}, s);
+      if (a.dissip_on) go_multi(L, M, MK_FACE3, FFaceRows<T, true, S>{1, (T)a.cd}, s);
+    } else if (L.face_rows) {
+      go_multi(L, M, MK_FACE3, FFaceRows<T, false, S>{a.dissip_on, (T)a.cd}, s);
+    } else if (a.dissip_on) {
+      go_multi(L, M, MK_FACE, FFace<T, S>{a.dissip_on, (T)a.cd}, s);
     } else {
-      go_multi(L, M, MK_PREP, FPrep<T, false>{a.dissip_on}, s);
-      if (a.dissip_on)
-        go_multi(L, M, MK_FACE, FFace<T>{a.dissip_on, (T)a.cd}, s);
-      else
-        go_multi(L, M, MK_FACE, FFaceConv<T>{}, s);
+      go_multi(L, M, MK_FACE, FFaceConv<T>{}, s);
     }
     go_multi(L, M, MK_REC, FRec<T>{a.dissip_on, (T)a.cd}, s);
     if (L.fast)
-      go_multi(L, M, MK_PHYS, FCombine<T, true>{a}, s);
+      go_multi(L, M, MK_PHYS, FCombine<T, true, S>{a}, s);
     else
-      go_multi(L, M, MK_PHYS, FCombine<T, false>{a}, s);
+      go_multi(L, M, MK_PHYS, FCombine<T, false, S>{a}, s);
     if (a.lres) return;
     if (a.irs) {
       if constexpr (std::is_same<T, double>::value) {
@@ -3633,7 +3810,7 @@ static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, b
         go_multi(L, M, MK_IRS1, FIrs<T, T, 1>{}, s);
         go_multi(L, M, MK_IRS2, FIrs<T, T, 2>{}, s);
       }
-      go_multi(L, M, MK_PHYS, FUpdate<T>{a}, s);
+      go_multi(L, M, MK_PHYS, FUpdate<T, S>{a}, s);
     }
     go_multi(L, M, MK_REC, FCutcell<T>{}, s);
     multi_bcond(L, M, s, a.faces_only && m < mstage);
@@ -3675,7 +3852,7 @@ void gather_residuals(const MultiLevel& L, double* res, unsigned* errs, cudaStre
 struct GroupEuler {
   const long long* off[MK_COUNT];
   long long tot[MK_COUNT];
-  int mstage, do_timestep, lfir, rt, fast, aux32;
+  int mstage, do_timestep, lfir, rt, fast, aux32, prep_rows, face_rows;
   StageArgs st[8];  // the stages (at most 8)
 };
 
@@ -3703,31 +3880,35 @@ __global__ void __launch_bounds__(256, 1) k_group_euler(MultiArgs<T> M, GroupEul
   if (G.do_timestep) {
     group_phase(M, G, MK_ONE, FDtimReset<T>{});
     grid.sync();
-    group_phase(M, G, MK_PHYS, FTimestep<T, TA>{});
+    group_phase(M, G, MK_PHYS, FTimestep<T, TA, false>{});
   }
   if (G.lfir) group_phase(M, G, MK_N5, FCopyWs<T>{});
   group_phase(M, G, MK_N, FSaveWn<T>{});
   grid.sync();
   for (int m = 1; m <= G.mstage; m++) {
     const StageArgs& a = G.st[m - 1];
+    if (G.prep_rows && G.fast)
+      group_phase(M, G, MK_PREP3, FPrepRows<T, true, false>{a.dissip_on});
+    else if (G.prep_rows)
+      group_phase(M, G, MK_PREP3, FPrepRows<T, false, false>{a.dissip_on});
+    else
+      group_phase(M, G, MK_PREP, FPrep<T, false, false>{a.dissip_on});
+    grid.sync();
     if (G.fast) {
-      group_phase(M, G, MK_PREP, FPrep<T, true>{a.dissip_on});
-      grid.sync();
-      if (a.dissip_on) group_phase(M, G, MK_FACE, FFaceDiss<T>{(T)a.cd});
+      if (a.dissip_on) group_phase(M, G, MK_FACE3, FFaceRows<T, true, false>{1, (T)a.cd});
+    } else if (G.face_rows) {
+      group_phase(M, G, MK_FACE3, FFaceRows<T, false, false>{a.dissip_on, (T)a.cd});
+    } else if (a.dissip_on) {
+      group_phase(M, G, MK_FACE, FFace<T, false>{a.dissip_on, (T)a.cd});
     } else {
-      group_phase(M, G, MK_PREP, FPrep<T, false>{a.dissip_on});
-      grid.sync();
-      if (a.dissip_on)
-        group_phase(M, G, MK_FACE, FFace<T>{a.dissip_on, (T)a.cd});
-      else
-        group_phase(M, G, MK_FACE, FFaceConv<T>{});
+      group_phase(M, G, MK_FACE, FFaceConv<T>{});
     }
     group_phase(M, G, MK_REC, FRec<T>{a.dissip_on, (T)a.cd});
     grid.sync();
     if (G.fast)
-      group_phase(M, G, MK_PHYS, FCombine<T, true>{a});
+      group_phase(M, G, MK_PHYS, FCombine<T, true, false>{a});
     else
-      group_phase(M, G, MK_PHYS, FCombine<T, false>{a});
+      group_phase(M, G, MK_PHYS, FCombine<T, false, false>{a});
     grid.sync();
     if (a.lres) return;
     if (a.irs) {
@@ -3745,7 +3926,7 @@ __global__ void __launch_bounds__(256, 1) k_group_euler(MultiArgs<T> M, GroupEul
         group_phase(M, G, MK_IRS2, FIrs<T, T, 2>{});
       }
       grid.sync();
-      group_phase(M, G, MK_PHYS, FUpdate<T>{a});
+      group_phase(M, G, MK_PHYS, FUpdate<T, false>{a});
       grid.sync();
     }
     group_phase(M, G, MK_REC, FCutcell<T>{});
@@ -3804,6 +3985,8 @@ static bool group_euler_coop(const MultiLevel& L, const StageArgs* A, int mstage
   G.rt = rt;
   G.fast = L.fast;
   G.aux32 = L.aux32;
+  G.prep_rows = L.prep_rows || (L.fast && L.coop);  // a contracted level always has the split scheme
+  G.face_rows = L.face_rows;
   for (int m = 0; m < mstage && m < 8; m++) G.st[m] = A[m];
   MultiArgs<T> M = multi_args<T>(L);
   const int grid = (int)std::max<long long>(1, std::min<long long>(most, gmax));
@@ -3824,9 +4007,11 @@ void multi_euler(const MultiLevel& L, const StageArgs* A, int mstage, bool with_
     if (done) return;
   }
   if (L.f32)
-    multi_euler_t<float>(L, A, mstage, with_timestep, lfir, rt, s);
+    multi_euler_t<float, true>(L, A, mstage, with_timestep, lfir, rt, s);
+  else if (L.tot[MK_PHYS] > kPlainCells)
+    multi_euler_t<double, true>(L, A, mstage, with_timestep, lfir, rt, s);
   else
-    multi_euler_t<double>(L, A, mstage, with_timestep, lfir, rt, s);
+    multi_euler_t<double, false>(L, A, mstage, with_timestep, lfir, rt, s);
 }
 
 template <typename TC, typename TF, typename F>
@@ -3910,6 +4095,7 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   template void launch_cutcell<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t);              \
   template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t, bool);                     \
   template long long bc_items<T>(const DevBlock<T>&, int);                                                      \
+  template long long split_items<T>(const DevBlock<T>&, int);                                                   \
   template void launch_rtrms<T>(const DevBlock<T>&, const PhysParams&, int, double*, int, double*, cudaStream_t, \
                                 unsigned*);                                                                    \
   template void launch_depvars_all<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                     \

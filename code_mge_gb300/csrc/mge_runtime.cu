@@ -1959,6 +1959,8 @@ void kind_counts(const Block& b, long long* n) {
   n[MK_PHYS] = nx * ny * nz;
   n[MK_PREP] = (nx + 2) * (ny + 2) * (nz + 2);
   n[MK_FACE] = (nx + 1) * (ny + 1) * (nz + 1);
+  n[MK_PREP3] = b.f32 ? split_items(b.dev32, 2) : split_items(b.dev, 2);
+  n[MK_FACE3] = b.f32 ? split_items(b.dev32, 1) : split_items(b.dev, 1);
   n[MK_N] = b.N;
   n[MK_N5] = 5 * b.N;
   n[MK_REC] = (long long)b.recs.size();
@@ -2064,6 +2066,7 @@ int build_plan(mge_ctx* const* cs, int n, int mlvl, GroupPlan** out, std::string
       rc = plan_upload(G, &L.off[m], off, why);
     }
     if (rc) return bad(rc);
+    split_passes(c0->P, L.fast, L.tot[MK_PHYS], &L.prep_rows, &L.face_rows);
     // small levels: the whole update of every case as one persistent
     // cooperative launch (MGE_GROUP_COOP_MAX_CELLS: the group's cells up to
     // which it does; 300,000 by default)
