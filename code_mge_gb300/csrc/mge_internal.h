@@ -128,6 +128,8 @@ enum : unsigned {
 struct IrsTables {
   const double* e1;   // pivot of row q (index 0..l)
   const double* e1r;  // RN(1/pivot)
+  const double* e1l;  // RN(1/pivot - e1r) or a neighbour: x/pivot = fma(x, e1r, x*e1l) when quick
+  int quick;          // that quotient rounds as the division for every pivot (quick_quotient)
   const double* e2;   // elimination factor
   // the same in single precision for the FP32 sweeps: the rounded pivot, the
   // single-precision RN(1/pivot) of that rounded pivot, the rounded factor

@@ -111,6 +111,12 @@ __device__ __forceinline__ double irs_e1(const IrsTables& t, int q, double) { re
 __device__ __forceinline__ float irs_e1(const IrsTables& t, int q, float) { return t.e1f[q]; }
 __device__ __forceinline__ double irs_e1r(const IrsTables& t, int q, double) { return t.e1r[q]; }
 __device__ __forceinline__ float irs_e1r(const IrsTables& t, int q, float) { return t.e1rf[q]; }
+// x / e1[q] as fma(x, e1r, x*e1l), with e1r + e1l = 1/e1 to twice the precision
+// (the host has checked that this rounds as the division for every x,
+// IrsTables::quick): one dependent operation fewer than Markstein's quotient
+template <bool SC> __device__ __forceinline__ double irs_quick(double x, double e1r, double e1l) {
+  return fma(x, e1r, SC ? smul(x, e1l) : x * e1l);
+}
 __device__ __forceinline__ double irs_e2(const IrsTables& t, int q, double) { return t.e2[q]; }
 __device__ __forceinline__ float irs_e2(const IrsTables& t, int q, float) { return t.e2f[q]; }
 template <typename T> __device__ __forceinline__ T fdimT(T a, T b) { return a > b ? a - b : T(0); }
@@ -1364,23 +1370,8 @@ __device__ __forceinline__ long long irs_lines(const DevBlock<T>& b) {
   return D == 0 ? (long long)b.ny * b.nz : (D == 1 ? (long long)b.nx * b.nz : (long long)b.nx * b.ny);
 }
 
-// the variable of (line, variable) item t: t / lines, which is 0..4
-__device__ __forceinline__ int line_var(long long t, long long lines) {
-  return (t >= lines) + (t >= 2 * lines) + (t >= 3 * lines) + (t >= 4 * lines);
-}
-
-// SC: the products of the forward and backward steps on the integer pipes.
-// That lengthens the serial chain of each line, so it pays only where many
-// lines run at once and the sweep is bound by the FP64 rate; with few lines
-// (coarse levels, slabs) the chain's latency bounds it and the FP64 forms
-// are faster.
-template <typename T, typename TC, int D, bool SC = false>
-__device__ __forceinline__ void body_irs(const DevBlock<T>& b, const IrsTables& tb, TC bb, long long t) {
-  const long long lines = irs_lines<T, D>(b);
-  const int v = line_var(t, lines);
-  const long long ln = t - (long long)v * lines;
-  long long c0, st;
-  int l;
+template <typename T, int D>
+__device__ __forceinline__ void line_of(const DevBlock<T>& b, long long ln, long long& c0, long long& st, int& l) {
   if (D == 0) {
     int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
     c0 = cidx(b.Pi, b.Pj, 0, j, k);
@@ -1397,14 +1388,46 @@ __device__ __forceinline__ void body_irs(const DevBlock<T>& b, const IrsTables& 
     st = (long long)b.Pi * b.Pj;
     l = b.kl;
   }
-  T* d = b.dw + (long long)v * b.N;
+}
+
+// the variable of (line, variable) item t: t / lines, which is 0..4
+__device__ __forceinline__ int line_var(long long t, long long lines) {
+  return (t >= lines) + (t >= 2 * lines) + (t >= 3 * lines) + (t >= 4 * lines);
+}
+
+// SC: the products of the forward and backward steps on the integer pipes.
+// That lengthens the serial chain of each line, so it pays only where many
+// lines run at once and the sweep is bound by the FP64 rate; with few lines
+// (coarse levels, slabs) the chain's latency bounds it and the FP64 forms
+// are faster.
+// QK: the quotient in two operations (irs_quick).
+// Every FP64 warp instruction takes 64 cycles of its scheduler, dependent or
+// not, whatever its active lanes, so a row costs 64 cycles an operation however
+// few the lines: 5 operations forward and 2 back with Markstein's quotient, 4 and
+// 2 with the short one, and every instruction around them adds to the chain.
+// A blanked row therefore keeps its value by a select, not a branch.  With the
+// short quotient, select and longer chunks, i and j sweeps: 512x512x2 202 and
+// 199 -> 162 and 151 us, 256x256x2 97 and 99 -> 79 and 78, 96^3 98 and 82 -> 90 and
+// 70, 192^3 569 and 381 -> 544 and 324.
+template <typename T, typename TC, int D, bool SC = false, bool QK = false, int K = 8>
+__device__ __forceinline__ void body_irs(const DevBlock<T>& b, const IrsTables& tb, TC bb, long long t) {
+  const long long lines = irs_lines<T, D>(b);
+  const int v = line_var(t, lines);
+  const long long ln = t - (long long)v * lines;
+  long long c0, st;
+  int l;
+  line_of<T, D>(b, ln, c0, st, l);
+  T* d = b.dw + (long long)v * b.N + c0;
+  const uint8_t* bl = b.blank + c0;
   TC prev;
   {
-    long long c = c0 + 2 * st;
-    TC x = (TC)d[c];
-    if (b.blank[c] != 0) {
-      x = x / irs_e1(tb, 2, TC(0));
-      d[c] = (T)x;
+    TC x = (TC)d[2 * st];
+    if (bl[2 * st] != 0) {
+      if constexpr (QK)
+        x = irs_quick<false>(x, tb.e1r[2], tb.e1l[2]);
+      else
+        x = x / irs_e1(tb, 2, TC(0));
+      d[2 * st] = (T)x;
     }
     prev = x;
   }
@@ -1412,50 +1435,65 @@ __device__ __forceinline__ void body_irs(const DevBlock<T>& b, const IrsTables& 
   // loaded before any of it is solved, so one memory latency is paid per
   // chunk instead of per cell.  Every cell is read once and written once
   // after its own read, so the order of results is unchanged.
-  constexpr int K = 8;
-  TC xb[K], pb[K], rb[K];
-  unsigned char bk[K];
-  for (int q0 = 3; q0 <= l; q0 += K) {
-#pragma unroll
-    for (int u = 0; u < K; u++)
-      if (q0 + u <= l) {
-        const long long c = c0 + (q0 + u) * st;
-        xb[u] = (TC)d[c];
-        bk[u] = b.blank[c];
+  constexpr bool tables_first = !(SC && D > 0);
+  auto forward = [&](int q0, auto whole) {
+    TC xb[K], pb[K], rb[K];
+    unsigned char bk[K];
+    // the tables with the chunk: behind the stores below they are loaded row
+    // by row, which the i sweep's strided lines and a warp alone on its
+    // scheduler wait for; many warps would rather have the registers
+    auto tables = [&](int u) {
+      if constexpr (QK)
+        pb[u] = tb.e1l[q0 + u];
+      else
         pb[u] = irs_e1(tb, q0 + u, TC(0));
-        rb[u] = irs_e1r(tb, q0 + u, TC(0));
+      rb[u] = irs_e1r(tb, q0 + u, TC(0));
+    };
+#pragma unroll
+    for (int u = 0; u < K; u++)
+      if (decltype(whole)::value || q0 + u <= l) {
+        xb[u] = (TC)d[(q0 + u) * st];
+        bk[u] = bl[(q0 + u) * st];
+        if (tables_first) tables(u);
       }
 #pragma unroll
     for (int u = 0; u < K; u++)
-      if (q0 + u <= l) {
-        TC x = xb[u];
-        if (bk[u] != 0) {
-          x = SC ? smdiv(x - smul(bb, prev), pb[u], rb[u]) : mdiv(x - bb * prev, pb[u], rb[u]);
-          d[c0 + (q0 + u) * st] = (T)x;
-        }
-        prev = x;
+      if (decltype(whole)::value || q0 + u <= l) {
+        if (!tables_first) tables(u);
+        const TC z = xb[u] - (SC ? smul(bb, prev) : bb * prev);
+        TC x;
+        if constexpr (QK)
+          x = irs_quick<SC>(z, rb[u], pb[u]);
+        else
+          x = SC ? smdiv(z, pb[u], rb[u]) : mdiv(z, pb[u], rb[u]);
+        prev = bk[u] != 0 ? x : xb[u];
+        if (bk[u] != 0) d[(q0 + u) * st] = (T)x;
       }
-  }
-  for (int q0 = l - 1; q0 >= 2; q0 -= K) {
+  };
+  int q0 = 3;
+  for (; q0 + K - 1 <= l; q0 += K) forward(q0, std::true_type{});
+  if (q0 <= l) forward(q0, std::false_type{});
+  auto backward = [&](int q0, auto whole) {
+    TC xb[K], pb[K];
+    unsigned char bk[K];
 #pragma unroll
     for (int u = 0; u < K; u++)
-      if (q0 - u >= 2) {
-        const long long c = c0 + (q0 - u) * st;
-        xb[u] = (TC)d[c];
-        bk[u] = b.blank[c];
+      if (decltype(whole)::value || q0 - u >= 2) {
+        xb[u] = (TC)d[(q0 - u) * st];
+        bk[u] = bl[(q0 - u) * st];
         pb[u] = irs_e2(tb, q0 - u, TC(0));
       }
 #pragma unroll
     for (int u = 0; u < K; u++)
-      if (q0 - u >= 2) {
-        TC x = xb[u];
-        if (bk[u] != 0) {
-          x = x - (SC ? smul(pb[u], prev) : pb[u] * prev);
-          d[c0 + (q0 - u) * st] = (T)x;
-        }
-        prev = x;
+      if (decltype(whole)::value || q0 - u >= 2) {
+        const TC x = xb[u] - (SC ? smul(pb[u], prev) : pb[u] * prev);
+        prev = bk[u] != 0 ? x : xb[u];
+        if (bk[u] != 0) d[(q0 - u) * st] = (T)x;
       }
-  }
+  };
+  q0 = l - 1;
+  for (; q0 - K + 1 >= 2; q0 -= K) backward(q0, std::true_type{});
+  if (q0 >= 2) backward(q0, std::false_type{});
 }
 
 // The FP32 sweeps of the mixed form's finest level, whose storage is FP64.
@@ -1523,14 +1561,9 @@ __device__ __forceinline__ void body_irs_mixed(const DevBlock<double>& b, const 
 #pragma unroll
     for (int u = 0; u < K; u++)
       if (q0 + u <= l) {
-        float x = xb[u];
-        if (bk[u] != 0) {
-          x = mdiv(x - bb * prev, pb[u], rb[u]);
-          m[c0 + (q0 + u) * st] = x;
-        } else if (fill) {
-          m[c0 + (q0 + u) * st] = x;
-        }
-        prev = x;
+        const float x = mdiv(xb[u] - bb * prev, pb[u], rb[u]);
+        prev = bk[u] != 0 ? x : xb[u];
+        if (fill || bk[u] != 0) m[c0 + (q0 + u) * st] = prev;
       }
   }
   // the backward pass does not revisit row l: its forward result is final
@@ -1547,12 +1580,9 @@ __device__ __forceinline__ void body_irs_mixed(const DevBlock<double>& b, const 
 #pragma unroll
     for (int u = 0; u < K; u++)
       if (q0 - u >= 2) {
-        float x = xb[u];
-        if (bk[u] != 0) {
-          x = x - pb[u] * prev;
-          o[c0 + (q0 - u) * st] = (TO)x;
-        }
-        prev = x;
+        const float x = xb[u] - pb[u] * prev;
+        prev = bk[u] != 0 ? x : xb[u];
+        if (bk[u] != 0) o[c0 + (q0 - u) * st] = (TO)x;
       }
   }
 }
@@ -1788,26 +1818,6 @@ size_t irs_smem_bytes(int len) {
 // pass through the stage scratch F, dead between the residual pass and the
 // next stage: slot q of a line holds progon3's v(q), w(q), u(q,1:5) on the
 // way forward and s(q-1), t(q-1,1:5) on the way back.
-template <typename T, int D>
-__device__ __forceinline__ void line_of(const DevBlock<T>& b, long long ln, long long& c0, long long& st, int& l) {
-  if (D == 0) {
-    int j = 2 + (int)((unsigned)ln % (unsigned)b.ny), k = 2 + (int)((unsigned)ln / (unsigned)b.ny);
-    c0 = cidx(b.Pi, b.Pj, 0, j, k);
-    st = 1;
-    l = b.il;
-  } else if (D == 1) {
-    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), k = 2 + (int)((unsigned)ln / (unsigned)b.nx);
-    c0 = cidx(b.Pi, b.Pj, i, 0, k);
-    st = b.Pi;
-    l = b.jl;
-  } else {
-    int i = 2 + (int)((unsigned)ln % (unsigned)b.nx), j = 2 + (int)((unsigned)ln / (unsigned)b.nx);
-    c0 = cidx(b.Pi, b.Pj, i, j, 0);
-    st = (long long)b.Pi * b.Pj;
-    l = b.kl;
-  }
-}
-
 template <typename T, typename TC, int D>
 __device__ __noinline__ void body_psmoo_line(const DevBlock<T>& b, long long ln) {
   const long long N = b.N;
@@ -2925,10 +2935,10 @@ __global__ void k_combine(DevBlock<T> b, PhysParams P, StageArgs A, unsigned* er
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST, S>(b, P, A, err, t);
 }
-template <typename T, typename TC, int D, bool SC = false>
+template <typename T, typename TC, int D, bool SC, bool QK, int K>
 __global__ void k_irs(DevBlock<T> b, IrsTables tb, TC bb) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < 5 * irs_lines<T, D>(b)) body_irs<T, TC, D, SC>(b, tb, bb, t);
+  if (t < 5 * irs_lines<T, D>(b)) body_irs<T, TC, D, SC, QK, K>(b, tb, bb, t);
 }
 template <typename T, bool S>
 __global__ void k_update(DevBlock<T> b, PhysParams P, StageArgs A) {
@@ -3174,7 +3184,14 @@ template <typename T, bool FAST, bool S> struct FCombine {
 template <typename T, typename TC, int D> struct FIrs {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < 5 * irs_lines<T, D>(b)) body_irs<T, TC, D>(b, M.tab[3 * q + D], (TC)(-M.P[q].smoo), t);
+    if (t >= 5 * irs_lines<T, D>(b)) return;
+    if constexpr (std::is_same<TC, double>::value) {
+      if (M.tab[3 * q + D].quick) {
+        body_irs<T, TC, D, false, true>(b, M.tab[3 * q + D], (TC)(-M.P[q].smoo), t);
+        return;
+      }
+    }
+    body_irs<T, TC, D>(b, M.tab[3 * q + D], (TC)(-M.P[q].smoo), t);
   }
 };
 // the mixed form's finest level: FP32 sweeps on one FP32 copy of dw (in F)
@@ -3445,10 +3462,18 @@ void launch_irs_dir(const DevBlock<T>& b, const IrsTables& tb, TC bb, cudaStream
     const long long grid = 5 * ((lines + LT - 1) / LT);
     k_irs_smem<T, TC, D, LT><<<(unsigned)grid, LT, sm, s>>>(b, tb, bb);
   } else {
-    if (5 * lines >= 150000)  // about 8 warps per scheduler: the sweep is bound by the FP64 rate
-      k_irs<T, TC, D, true><<<LAUNCH_N(5 * lines), 0, s>>>(b, tb, bb);
-    else
-      k_irs<T, TC, D><<<LAUNCH_N(5 * lines), 0, s>>>(b, tb, bb);
+    const auto go = [&](auto QK) {
+      if (5 * lines >= 150000)  // about 8 warps per scheduler: the sweep is bound by the FP64 rate
+        k_irs<T, TC, D, true, QK.value, 8><<<LAUNCH_N(5 * lines), 0, s>>>(b, tb, bb);
+      else if (5 * lines <= 8192)  // under half the schedulers have a warp: the memory latency a chunk pays shows
+        k_irs<T, TC, D, false, QK.value, 24><<<LAUNCH_N(5 * lines), 0, s>>>(b, tb, bb);
+      else
+        k_irs<T, TC, D, false, QK.value, 8><<<LAUNCH_N(5 * lines), 0, s>>>(b, tb, bb);
+    };
+    if constexpr (std::is_same<TC, double>::value) {
+      if (tb.quick) return go(std::true_type{});
+    }
+    go(std::false_type{});
   }
 }
 

@@ -21,6 +21,7 @@
 
 #include "../../include/mge_gpu.h"
 #include "mge_internal.h"
+#include "quick_quotient.h"
 
 using namespace mge;
 
@@ -678,10 +679,10 @@ int commit_block(mge_ctx* c, Block& b, double* scratch) {
   // IRS tables
   const int lens[3] = {b.il, b.jl, b.kl}, lms[3] = {b.nx, b.ny, b.nz};
   size_t tot = 0;
-  for (int d = 0; d < 3; d++) tot += 3 * (size_t)(lens[d] + 2);
+  for (int d = 0; d < 3; d++) tot += 4 * (size_t)(lens[d] + 2);
   if ((rc = dalloc(c, &b.irs, tot))) return rc;
   std::vector<double> all;
-  size_t offs[3][3];
+  size_t offs[3][4];
   for (int d = 0; d < 3; d++) {
     std::vector<double> e1, e1r, e2;
     irs_pivots(c->prm.smoo > 0.0 ? c->prm.smoo : 0.0, lms[d], lens[d], e1, e1r, e2);
@@ -691,6 +692,16 @@ int commit_block(mge_ctx* c, Block& b, double* scratch) {
     all.insert(all.end(), e1r.begin(), e1r.end());
     offs[d][2] = all.size();
     all.insert(all.end(), e2.begin(), e2.end());
+    std::vector<double> low(e1.size(), 0.0);
+    b.tabs[d].quick = 1;
+    for (int q = 2; q <= lens[d]; q++) {
+      if (q > 2 && e1[q] == e1[q - 1])
+        low[q] = low[q - 1];
+      else if (!quick_quotient(e1[q], e1r[q], &low[q]))
+        b.tabs[d].quick = 0;
+    }
+    offs[d][3] = all.size();
+    all.insert(all.end(), low.begin(), low.end());
   }
   CK(cudaMemcpy(b.irs, all.data(), all.size() * 8, cudaMemcpyHostToDevice));
   // single-precision tables: the FP32 sweeps then need no conversion per cell
@@ -704,6 +715,7 @@ int commit_block(mge_ctx* c, Block& b, double* scratch) {
     b.tabs[d].e1 = b.irs + offs[d][0];
     b.tabs[d].e1r = b.irs + offs[d][1];
     b.tabs[d].e2 = b.irs + offs[d][2];
+    b.tabs[d].e1l = b.irs + offs[d][3];
     b.tabs[d].e1f = b.irs32 + offs[d][0];
     b.tabs[d].e1rf = b.irs32 + offs[d][1];
     b.tabs[d].e2f = b.irs32 + offs[d][2];
