@@ -270,21 +270,15 @@ template <typename T> __global__ void k_dtim_convert(double* src, T* dst) {
 
 // --------------------------------------------------------------- stage: per-cell pass
 // Box [1..ie]x[1..je]x[1..ke]: every cell whose flux or sensor a face needs.
-template <typename T>
+template <bool S, typename T>
 __device__ __forceinline__ T van_albada(T a, T b, T e2);
 
-// SLOPES: the MUSCL Roe form with the velocities of every cell already in
-// F[0..2] (k_prim): the limited slope of each primitive variable along each
-// direction goes to dlt[dir][var], once per cell.  A face takes the slope of
-// its lower cell for the left state and that of its upper cell for the right
-// state, the same van_albada(q(c)-q(c-1), q(c+1)-q(c)) it would form itself.
-//
 // FAST: the contracted form of the mixed precision's finest level (JST
 // central scheme, Euler): the cell flux takes the velocity q = (w_d s)/rho
 // once and multiplies, F(v) = q w(v), instead of rounding each product
 // before its division.  The result is the same quantity to an FP64 rounding
 // or two, not the reference's bit pattern.
-template <typename T, bool SLOPES = false, bool FAST = false, bool S = true>
+template <typename T, bool FAST = false, bool S = true>
 __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams& P, int dissip_on, long long t) {
   const int ex = b.ie, ey = b.je;  // count = ie (cells 1..ie)
   int i, j, k;
@@ -303,26 +297,6 @@ __device__ __forceinline__ void body_prep(const DevBlock<T>& b, const PhysParams
 #pragma unroll
     for (int a = 0; a < 3; a++) b.vt[a * N + c] = solid ? T(0) : mdiv(w[1 + a], w[0], y);
     b.vt[3 * N + c] = solid ? T(0) : pdiv<S>(p, w[0] * (T)P.gas_const);
-  }
-  if (SLOPES) {
-    const long long sts[3] = {1, (long long)b.Pi, (long long)b.Pi * b.Pj};
-    // a face along d has physical tangential indices: only those cells need
-    // the slope along d
-    const bool ti = i >= 2 && i <= b.il, tj = j >= 2 && j <= b.jl, tk = k >= 2 && k <= b.kl;
-    const bool need[3] = {tj && tk, ti && tk, ti && tj};
-    auto prim = [&](long long q, int v) -> T {
-      return v == 0 ? b.w[q] : (v == 4 ? b.p[q] : b.F[(long long)(v - 1) * N + q]);
-    };
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      if (!need[d]) continue;
-#pragma unroll
-      for (int v = 0; v < 5; v++) {
-        const T q0 = prim(c, v);
-        const T dm = q0 - prim(c - sts[d], v), dp = prim(c + sts[d], v) - q0;
-        b.dlt[(long long)(d * 5 + v) * N + c] = van_albada(dm, dp, (T)P.lim_e2[v]);
-      }
-    }
   }
   // the MUSCL Roe faces take their central flux from the reconstructed
   // states, not from the cell fluxes
@@ -496,66 +470,80 @@ __device__ __noinline__ void dflux_matrix(T gamma, const T* u1, const T* u2, con
 // (the reference's roepak/viscpak sources are not in its tree; these follow
 // the published methods, as the oracle does: Roe 1981 with Harten's entropy
 // fix, MUSCL with the van Albada limiter, central-gradient laminar stresses)
-template <typename T>
+template <bool S, typename T>
 __device__ __forceinline__ T van_albada(T a, T b, T e2) {
   // smooth form, no cut-off at a*b <= 0: with e2 > 0 a cut-off would make the
   // slope jump by up to b/3 when a changes sign.  Both differences zero (a
   // uniform stretch) and e2 > 0: the numerator is e2*a + e2*b, a zero with
   // the sign of a + b, and so is the quotient
   if (a == T(0) && b == T(0) && e2 > T(0)) return a + b;
-  return sdiv((b * b + e2) * a + (a * a + e2) * b, a * a + b * b + T(2) * e2);
+  const T aa = pmul<S>(a, a), bb = pmul<S>(b, b);
+  return pdiv<S>(pmul<S>(bb + e2, a) + pmul<S>(aa + e2, b), aa + bb + mul2(e2));
 }
 
 // yl, yr: RN(1/wl[0]) and RN(1/wr[0]); every quotient below that shares a
 // divisor takes one reciprocal and mdiv, which rounds as the division does
-template <typename T>
-__device__ __noinline__ void roe_diss(const PhysParams& P, int d, T S, const T* wl, T pl, const T* wr, T pr, T yl, T yr,
-                                      T* out) {
+template <typename T, bool S>
+__device__ __forceinline__ void roe_diss_inl(const PhysParams& P, int d, T area, const T* wl, T pl, const T* wr, T pr,
+                                             T yl, T yr, T* out) {
   const T g = (T)P.gamma;
   T ul[3], ur[3];
+#pragma unroll
   for (int a = 0; a < 3; a++) {
-    ul[a] = mdiv(wl[1 + a], wl[0], yl);
-    ur[a] = mdiv(wr[1 + a], wr[0], yr);
+    ul[a] = pmdiv<S>(wl[1 + a], wl[0], yl);
+    ur[a] = pmdiv<S>(wr[1 + a], wr[0], yr);
   }
-  T hl = mdiv(wl[4] + pl, wl[0], yl), hr = mdiv(wr[4] + pr, wr[0], yr);
-  T rt = sqrt(mdiv(wr[0], wl[0], yl));
-  T rh = rt * wl[0];
-  const T den = T(1) + rt, yden = sdiv(T(1), den);
+  const T hl = pmdiv<S>(wl[4] + pl, wl[0], yl), hr = pmdiv<S>(wr[4] + pr, wr[0], yr);
+  const T rt = sqrt(pmdiv<S>(wr[0], wl[0], yl));
+  const T rh = pmul<S>(rt, wl[0]);
+  const T den = T(1) + rt, yden = pdiv<S>(T(1), den);
   T uh[3];
-  for (int a = 0; a < 3; a++) uh[a] = mdiv(ul[a] + rt * ur[a], den, yden);
-  T hh = mdiv(hl + rt * hr, den, yden);
-  T q2 = uh[0] * uh[0] + uh[1] * uh[1] + uh[2] * uh[2];
-  T c2 = (g - T(1)) * (hh - T(0.5) * q2);
-  T ch = sqrt(fmaxT(c2, (T)1e-300));
-  T un = uh[d];
-  T dr = wr[0] - wl[0], dp = pr - pl, dun = ur[d] - ul[d];
-  T du[3] = {ur[0] - ul[0], ur[1] - ul[1], ur[2] - ul[2]};
-  T delta = (T)P.epsentr * (fabs(un) + ch);
+#pragma unroll
+  for (int a = 0; a < 3; a++) uh[a] = pmdiv<S>(ul[a] + pmul<S>(rt, ur[a]), den, yden);
+  const T hh = pmdiv<S>(hl + pmul<S>(rt, hr), den, yden);
+  const T q2 = pmul<S>(uh[0], uh[0]) + pmul<S>(uh[1], uh[1]) + pmul<S>(uh[2], uh[2]);
+  const T c2 = pmul<S>(g - T(1), hh - mulhalf(q2));
+  const T ch = sqrt(fmaxT(c2, (T)1e-300));
+  const T un = d == 0 ? uh[0] : (d == 1 ? uh[1] : uh[2]);
+  const T dr = wr[0] - wl[0], dp = pr - pl;
+  T du[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) du[a] = ur[a] - ul[a];
+  const T dun = d == 0 ? du[0] : (d == 1 ? du[1] : du[2]);
+  const T delta = pmul<S>((T)P.epsentr, fabs(un) + ch);
   auto fix = [&](T lam) {
-    T a = fabs(lam);
-    return (a < delta && delta > T(0)) ? sdiv(lam * lam + delta * delta, T(2) * delta) : a;
+    const T a = fabs(lam);
+    return (a < delta && delta > T(0)) ? pdiv<S>(pmul<S>(lam, lam) + pmul<S>(delta, delta), mul2(delta)) : a;
   };
-  T l1 = fix(un - ch), l2 = fix(un), l5 = fix(un + ch);
-  const T c22 = T(2) * c2, yc22 = sdiv(T(1), c22);
-  T a1 = mdiv(dp - rh * ch * dun, c22, yc22);
-  T a2 = dr - sdiv(dp, c2);
-  T a5 = mdiv(dp + rh * ch * dun, c22, yc22);
+  const T l1 = fix(un - ch), l2 = fix(un), l5 = fix(un + ch);
+  const T c22 = mul2(c2), yc22 = pdiv<S>(T(1), c22);
+  const T rcd = pmul<S>(pmul<S>(rh, ch), dun);
+  const T a1 = pmdiv<S>(dp - rcd, c22, yc22);
+  const T a2 = dr - pdiv<S>(dp, c2);
+  const T a5 = pmdiv<S>(dp + rcd, c22, yc22);
+  const T w1 = pmul<S>(l1, a1), w5 = pmul<S>(l5, a5);
   T sh[3];
-  for (int a = 0; a < 3; a++) sh[a] = rh * (du[a] - (a == d ? dun : T(0)));
-  T k1[5], k5[5];
-  k1[0] = T(1);
-  k5[0] = T(1);
-  for (int a = 0; a < 3; a++) {
-    k1[1 + a] = uh[a] - (a == d ? ch : T(0));
-    k5[1 + a] = uh[a] + (a == d ? ch : T(0));
-  }
-  k1[4] = hh - ch * un;
-  k5[4] = hh + ch * un;
+#pragma unroll
+  for (int a = 0; a < 3; a++) sh[a] = pmul<S>(rh, du[a] - (a == d ? dun : T(0)));
   T res[5];
-  res[0] = l1 * a1 * k1[0] + l2 * a2 + l5 * a5 * k5[0];
-  for (int a = 0; a < 3; a++) res[1 + a] = l1 * a1 * k1[1 + a] + l2 * (a2 * uh[a] + sh[a]) + l5 * a5 * k5[1 + a];
-  res[4] = l1 * a1 * k1[4] + l2 * (a2 * T(0.5) * q2 + (uh[0] * sh[0] + uh[1] * sh[1] + uh[2] * sh[2])) + l5 * a5 * k5[4];
-  for (int v = 0; v < 5; v++) out[v] = T(0.5) * S * res[v];
+  res[0] = w1 + pmul<S>(l2, a2) + w5;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const T k1 = uh[a] - (a == d ? ch : T(0)), k5 = uh[a] + (a == d ? ch : T(0));
+    res[1 + a] = pmul<S>(w1, k1) + pmul<S>(l2, pmul<S>(a2, uh[a]) + sh[a]) + pmul<S>(w5, k5);
+  }
+  const T cu = pmul<S>(ch, un);
+  const T en = pmul<S>(mulhalf(a2), q2) + (pmul<S>(uh[0], sh[0]) + pmul<S>(uh[1], sh[1]) + pmul<S>(uh[2], sh[2]));
+  res[4] = pmul<S>(w1, hh - cu) + pmul<S>(l2, en) + pmul<S>(w5, hh + cu);
+  const T ha = mulhalf(area);
+#pragma unroll
+  for (int v = 0; v < 5; v++) out[v] = pmul<S>(ha, res[v]);
+}
+
+template <typename T, bool S>
+__device__ __noinline__ void roe_diss(const PhysParams& P, int d, T area, const T* wl, T pl, const T* wr, T pr, T yl, T yr,
+                                      T* out) {
+  roe_diss_inl<T, S>(P, d, area, wl, pl, wr, pr, yl, yr, out);
 }
 
 // face q (between q-1 and q) along D at cell c: cell states, MUSCL when order 2
@@ -586,8 +574,8 @@ __device__ __noinline__ void face_states(const DevBlock<T>& b, const PhysParams&
   for (int kq = 0; kq < 5; kq++) {
     T dm = qv[1][kq] - qv[0][kq], d0 = qv[2][kq] - qv[1][kq], dp = qv[3][kq] - qv[2][kq];
     T e2 = (T)P.lim_e2[kq];
-    L[kq] = qv[1][kq] + T(0.5) * van_albada(dm, d0, e2);
-    R[kq] = qv[2][kq] - T(0.5) * van_albada(d0, dp, e2);
+    L[kq] = qv[1][kq] + T(0.5) * van_albada<true>(dm, d0, e2);
+    R[kq] = qv[2][kq] - T(0.5) * van_albada<true>(d0, dp, e2);
   }
   if (L[0] <= T(0) || R[0] <= T(0) || L[4] <= T(0) || R[4] <= T(0)) return;
   const T gm1 = (T)P.gamma - T(1), rg = rcp_gm1(P, T(0));
@@ -607,8 +595,8 @@ __device__ __noinline__ void face_states(const DevBlock<T>& b, const PhysParams&
 // face_states in the MUSCL form from the per-cell velocities (F[0..2]) and
 // limited slopes (dlt) of k_prim and the prep pass: the same values, with each
 // quotient and slope formed once per cell instead of once per face
-template <typename T, int D>
-__device__ __noinline__ void face_states_pre(const DevBlock<T>& b, const PhysParams& P, long long c, int q, T* wl, T* pl,
+template <typename T, int D, bool S>
+__device__ __forceinline__ void face_states_pre(const DevBlock<T>& b, const PhysParams& P, long long c, int q, T* wl, T* pl,
                                              T* wr, T* pr) {
   const long long N = b.N;
   const long long st = D == 0 ? 1 : (D == 1 ? (long long)b.Pi : (long long)b.Pi * b.Pj);
@@ -622,44 +610,46 @@ __device__ __noinline__ void face_states_pre(const DevBlock<T>& b, const PhysPar
   const int lq = D == 0 ? b.il : (D == 1 ? b.jl : b.kl);
   if (q - 2 < 0 || q + 1 > lq + 2) return;
   if (b.blank[c - 2 * st] == 0 || b.blank[cm] == 0 || b.blank[c] == 0 || b.blank[c + st] == 0) return;
-  const T* S = b.dlt + (long long)(D * 5) * N;
+  const T* sl = b.dlt + (long long)(D * 5) * N;
   T L[5], R[5];
-  L[0] = wl[0] + T(0.5) * S[cm];
-  R[0] = wr[0] - T(0.5) * S[c];
+  L[0] = wl[0] + mulhalf(sl[cm]);
+  R[0] = wr[0] - mulhalf(sl[c]);
   for (int a = 0; a < 3; a++) {
-    L[1 + a] = b.F[(long long)a * N + cm] + T(0.5) * S[(long long)(1 + a) * N + cm];
-    R[1 + a] = b.F[(long long)a * N + c] - T(0.5) * S[(long long)(1 + a) * N + c];
+    L[1 + a] = b.F[(long long)a * N + cm] + mulhalf(sl[(long long)(1 + a) * N + cm]);
+    R[1 + a] = b.F[(long long)a * N + c] - mulhalf(sl[(long long)(1 + a) * N + c]);
   }
-  L[4] = *pl + T(0.5) * S[4 * N + cm];
-  R[4] = *pr - T(0.5) * S[4 * N + c];
+  L[4] = *pl + mulhalf(sl[4 * N + cm]);
+  R[4] = *pr - mulhalf(sl[4 * N + c]);
   if (L[0] <= T(0) || R[0] <= T(0) || L[4] <= T(0) || R[4] <= T(0)) return;
   const T gm1 = (T)P.gamma - T(1), rg = rcp_gm1(P, T(0));
   wl[0] = L[0];
   wr[0] = R[0];
   for (int a = 0; a < 3; a++) {
-    wl[1 + a] = L[0] * L[1 + a];
-    wr[1 + a] = R[0] * R[1 + a];
+    wl[1 + a] = pmul<S>(L[0], L[1 + a]);
+    wr[1 + a] = pmul<S>(R[0], R[1 + a]);
   }
-  wl[4] = mdiv(L[4], gm1, rg) + T(0.5) * L[0] * (L[1] * L[1] + L[2] * L[2] + L[3] * L[3]);
-  wr[4] = mdiv(R[4], gm1, rg) + T(0.5) * R[0] * (R[1] * R[1] + R[2] * R[2] + R[3] * R[3]);
+  wl[4] = pmdiv<S>(L[4], gm1, rg) +
+          pmul<S>(mulhalf(L[0]), pmul<S>(L[1], L[1]) + pmul<S>(L[2], L[2]) + pmul<S>(L[3], L[3]));
+  wr[4] = pmdiv<S>(R[4], gm1, rg) +
+          pmul<S>(mulhalf(R[0]), pmul<S>(R[1], R[1]) + pmul<S>(R[2], R[2]) + pmul<S>(R[3], R[3]));
   *pl = L[4];
   *pr = R[4];
 }
 
-template <typename T>
+template <bool S, typename T>
 __device__ __forceinline__ void ceflux_gen(int D, const T* w, T p, T s, T y, T* f) {
-  T f0 = w[1 + D] * s;
+  T f0 = pmul<S>(w[1 + D], s);
   f[0] = f0;
-  f[1] = mdiv(f0 * w[1], w[0], y);
-  f[2] = mdiv(f0 * w[2], w[0], y);
-  f[3] = mdiv(f0 * w[3], w[0], y);
-  f[1 + D] = f[1 + D] + p * s;
-  f[4] = mdiv(f0 * (w[4] + p), w[0], y);
+  f[1] = pmdiv<S>(pmul<S>(f0, w[1]), w[0], y);
+  f[2] = pmdiv<S>(pmul<S>(f0, w[2]), w[0], y);
+  f[3] = pmdiv<S>(pmul<S>(f0, w[3]), w[0], y);
+  f[1 + D] = f[1 + D] + pmul<S>(p, s);
+  f[4] = pmdiv<S>(pmul<S>(f0, w[4] + p), w[0], y);
 }
 
 // laminar viscous flux through face q along D (at cell c), times S
-template <typename T, int D>
-__device__ __noinline__ void visc_face(const DevBlock<T>& b, const PhysParams& P, long long c, T S, T* out) {
+template <typename T, int D, bool S>
+__device__ __forceinline__ void visc_face_inl(const DevBlock<T>& b, const PhysParams& P, long long c, T area, T* out) {
   const long long N = b.N;
   const long long st[3] = {1, (long long)b.Pi, (long long)b.Pi * b.Pj};
   const long long cl = c - st[D];
@@ -669,21 +659,27 @@ __device__ __noinline__ void visc_face(const DevBlock<T>& b, const PhysParams& P
     const T* f = b.vt + (long long)a * N;
     for (int t = 0; t < 3; t++) {
       if (t == D)
-        g[a][t] = mdiv(f[c] - f[cl], (T)h[D], rcp_h(b, D));
+        g[a][t] = pmdiv<S>(f[c] - f[cl], (T)h[D], rcp_h(b, D));
       else
-        g[a][t] = mdiv((f[c + st[t]] - f[c - st[t]]) + (f[cl + st[t]] - f[cl - st[t]]), T(4) * (T)h[t],
+        g[a][t] = pmdiv<S>((f[c + st[t]] - f[c - st[t]]) + (f[cl + st[t]] - f[cl - st[t]]), T(4) * (T)h[t],
                        rcp_4h(b, t));
     }
   }
   const T mu = (T)P.viscl, kt = (T)P.kt;
   T div = g[0][0] + g[1][1] + g[2][2];
   T tau[3];
-  for (int a = 0; a < 3; a++) tau[a] = mu * (g[a][D] + g[D][a]) - (a == D ? (T(2) / T(3)) * mu * div : T(0));
+  for (int a = 0; a < 3; a++)
+    tau[a] = pmul<S>(mu, g[a][D] + g[D][a]) - (a == D ? pmul<S>((T(2) / T(3)) * mu, div) : T(0));
   T uf[3];
-  for (int a = 0; a < 3; a++) uf[a] = T(0.5) * (b.vt[a * N + cl] + b.vt[a * N + c]);
+  for (int a = 0; a < 3; a++) uf[a] = mulhalf(b.vt[a * N + cl] + b.vt[a * N + c]);
   out[0] = T(0);
-  for (int a = 0; a < 3; a++) out[1 + a] = S * tau[a];
-  out[4] = S * ((uf[0] * tau[0] + uf[1] * tau[1] + uf[2] * tau[2]) + kt * g[3][D]);
+  for (int a = 0; a < 3; a++) out[1 + a] = pmul<S>(area, tau[a]);
+  out[4] = pmul<S>(area, (pmul<S>(uf[0], tau[0]) + pmul<S>(uf[1], tau[1]) + pmul<S>(uf[2], tau[2])) + pmul<S>(kt, g[3][D]));
+}
+
+template <typename T, int D, bool S>
+__device__ __noinline__ void visc_face(const DevBlock<T>& b, const PhysParams& P, long long c, T area, T* out) {
+  visc_face_inl<T, D, S>(b, P, c, area, out);
 }
 
 // --------------------------------------------------------------- stage: per-face pass
@@ -706,36 +702,42 @@ __device__ __forceinline__ void face_dir(const DevBlock<T>& b, const PhysParams&
   T* E = b.efs + (long long)(D * 5) * N;
   if (SCH != FACE_JST && P.eqn_ns && dissip_on) {  // viscous face flux, blended like the dissipation
     T o[5];
-    visc_face<T, D>(b, P, c, (T)fabs(b.s[D]), o);
+    if (SCH == FACE_ROE)
+      visc_face_inl<T, D, S>(b, P, c, (T)fabs(b.s[D]), o);
+    else
+      visc_face<T, D, S>(b, P, c, (T)fabs(b.s[D]), o);
     T* V = b.vfs + (long long)(D * 5) * N;
 #pragma unroll
-    for (int v = 0; v < 5; v++) V[v * N + c] = cd * o[v];
+    for (int v = 0; v < 5; v++) V[v * N + c] = pmul<S>(cd, o[v]);
   }
   const bool roe = SCH == FACE_ROE || (SCH == FACE_ANY && P.distype != 0);
   if (roe) {  // Roe: central part of the (reconstructed) states, upwind part into dfs
     T wl[5], wr[5], pl, pr;
     if (SCH == FACE_ROE && P.distype == 2)
-      face_states_pre<T, D>(b, P, c, q, wl, &pl, wr, &pr);
+      face_states_pre<T, D, S>(b, P, c, q, wl, &pl, wr, &pr);
     else
       face_states<T, D>(b, P, c, q, P.distype == 2 ? 2 : 1, wl, &pl, wr, &pr);
     const T yl = pdiv<S>(T(1), wl[0]), yr = pdiv<S>(T(1), wr[0]);
     if (P.distype == 2) {
       T f1[5], f2[5];
-      ceflux_gen<T>(D, wr, pr, (T)b.s[D], yr, f1);
-      ceflux_gen<T>(D, wl, pl, (T)b.s[D], yl, f2);
+      ceflux_gen<S, T>(D, wr, pr, (T)b.s[D], yr, f1);
+      ceflux_gen<S, T>(D, wl, pl, (T)b.s[D], yl, f2);
 #pragma unroll
-      for (int v = 0; v < 5; v++) E[v * N + c] = T(0.5) * (f1[v] + f2[v]);
+      for (int v = 0; v < 5; v++) E[v * N + c] = mulhalf(f1[v] + f2[v]);
     } else {
       const T* F = b.F + (long long)(D * 5) * N;
 #pragma unroll
-      for (int v = 0; v < 5; v++) E[v * N + c] = T(0.5) * (F[v * N + c] + F[v * N + c - st]);
+      for (int v = 0; v < 5; v++) E[v * N + c] = mulhalf(F[v * N + c] + F[v * N + c - st]);
     }
     if (!dissip_on) return;
     T o[5];
-    roe_diss<T>(P, D, (T)fabs(b.s[D]), wl, pl, wr, pr, yl, yr, o);
+    if (SCH == FACE_ROE)
+      roe_diss_inl<T, S>(P, D, (T)fabs(b.s[D]), wl, pl, wr, pr, yl, yr, o);
+    else
+      roe_diss<T, S>(P, D, (T)fabs(b.s[D]), wl, pl, wr, pr, yl, yr, o);
     T* Df = b.dfs + (long long)(D * 5) * N;
 #pragma unroll
-    for (int v = 0; v < 5; v++) Df[v * N + c] = cd * o[v];
+    for (int v = 0; v < 5; v++) Df[v * N + c] = pmul<S>(cd, o[v]);
     return;
   }
   // convective: efs(q) = 0.5*(F(q) + F(q-1))
@@ -844,7 +846,7 @@ __device__ __forceinline__ void face_diss_fast(const DevBlock<T>& b, const PhysP
 
 // One direction of the face pass, at the faces along D between physical lines
 // of cells; FAST: the contracted form's dissipation faces
-template <typename T, bool FAST, bool S, int D>
+template <typename T, bool FAST, bool S, int D, int SCH = FACE_JST>
 __device__ __forceinline__ void body_face_split(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd, int t) {
   const int n0 = b.nx + (D == 0), n1 = b.ny + (D == 1), n2 = b.nz + (D == 2);
   if (t >= n0 * n1 * n2) return;
@@ -853,7 +855,7 @@ __device__ __forceinline__ void body_face_split(const DevBlock<T>& b, const Phys
   if (FAST)
     face_diss_fast<T, D, S>(b, P, cd, i, j, k);
   else
-    face_dir<T, D, FACE_JST, S>(b, P, dissip_on, cd, i, j, k);
+    face_dir<T, D, SCH, S>(b, P, dissip_on, cd, i, j, k);
 }
 
 // The split passes as one range of items: three rows, one per direction, each
@@ -962,9 +964,9 @@ __device__ void rec_wall_terms(const DevBlock<T>& b, const PhysParams& P, int di
     const T S = (T)fabs(b.s[D]);
     const T yc = T(1) / wc[0], ys = T(1) / wsol[0];
     if (plus)
-      roe_diss<T>(P, D, S, wc, b.p[c], wsol, psol, yc, ys, o);
+      roe_diss<T, false>(P, D, S, wc, b.p[c], wsol, psol, yc, ys, o);
     else
-      roe_diss<T>(P, D, S, wsol, psol, wc, b.p[c], ys, yc, o);
+      roe_diss<T, false>(P, D, S, wsol, psol, wc, b.p[c], ys, yc, o);
     for (int v = 0; v < 5; v++) W[15 + v] = plus ? -(cd * o[v]) : cd * o[v];
     return;
   }
@@ -2856,21 +2858,61 @@ __global__ void k_forces(DevBlock<T> b, double ox, double oy, double oz, double 
 }
 
 // =============================================================== one-launch-per-phase kernels
-template <typename T, bool SLOPES, bool FAST, bool S>
-__global__ void __launch_bounds__(256, SLOPES ? 3 : (S ? 6 : 4)) k_prep(DevBlock<T> b, PhysParams P, int dissip_on) {
+template <typename T, bool FAST, bool S>
+__global__ void __launch_bounds__(256, S ? 6 : 4) k_prep(DevBlock<T> b, PhysParams P, int dissip_on) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)b.ie * b.je * b.ke) body_prep<T, SLOPES, FAST, S>(b, P, dissip_on, t);
+  if (t < (long long)b.ie * b.je * b.ke) body_prep<T, FAST, S>(b, P, dissip_on, t);
 }
-// the velocities of every cell, ghosts included, into F[0..2] for the MUSCL
-// Roe form (one reciprocal of the density and mdiv: the IEEE quotients)
-template <typename T>
-__global__ void k_prim(DevBlock<T> b) {
+// The MUSCL Roe form's prep pass, in two.  First the velocities of every cell,
+// ghosts included, into F[0..2] (one reciprocal of the density and mdiv: the
+// IEEE quotients); with NS also the velocities and temperature of the viscous
+// faces, zero in solid cells (euler.f90:140-154).
+template <typename T, bool S>
+__global__ void k_prim(DevBlock<T> b, PhysParams P, int dissip_on) {
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= b.N) return;
   const long long N = b.N;
-  const T r = b.w[c], y = T(1) / r;
+  const T r = b.w[c], y = pdiv<S>(T(1), r);
+  const bool visc = P.eqn_ns && dissip_on, solid = visc && b.blank[c] == 0;
 #pragma unroll
-  for (int a = 0; a < 3; a++) b.F[(long long)a * N + c] = mdiv(b.w[(long long)(1 + a) * N + c], r, y);
+  for (int a = 0; a < 3; a++) {
+    const T u = pmdiv<S>(b.w[(long long)(1 + a) * N + c], r, y);
+    b.F[(long long)a * N + c] = u;
+    if (visc) b.vt[a * N + c] = solid ? T(0) : u;
+  }
+  if (visc) b.vt[3 * N + c] = solid ? T(0) : pdiv<S>(b.p[c], pmul<S>(r, (T)P.gas_const));
+}
+// Then the limited slope of each primitive variable along each direction,
+// once per cell, into dlt[dir][var].  A face takes the slope of its lower cell
+// for the left state and that of its upper cell for the right state, the same
+// van_albada(q(c)-q(c-1), q(c+1)-q(c)) it would form itself.  One direction per
+// grid row, at the cells a face along it reads (tangential indices physical).
+// The whole-cell pass took 350-530 us at 512x512x2 (the less, the more of the level
+// is uniform), the two take 280-420.
+template <typename T, bool S, int D>
+__device__ __forceinline__ void body_slopes(const DevBlock<T>& b, const PhysParams& P, int t) {
+  const int n0 = b.nx + (D == 0 ? 2 : 0), n1 = b.ny + (D == 1 ? 2 : 0), n2 = b.nz + (D == 2 ? 2 : 0);
+  if (t >= n0 * n1 * n2) return;
+  int i, j, k;
+  cell_of(t, n0, n1, 2, i, j, k);
+  if (D == 0) i -= 1;
+  if (D == 1) j -= 1;
+  if (D == 2) k -= 1;
+  const long long N = b.N, st = D == 0 ? 1 : (D == 1 ? (long long)b.Pi : (long long)b.Pi * b.Pj);
+  const long long c = cidx(b.Pi, b.Pj, i, j, k);
+  const T* prim[5] = {b.w, b.F, b.F + N, b.F + 2 * N, b.p};
+#pragma unroll
+  for (int v = 0; v < 5; v++) {
+    const T q0 = prim[v][c], dm = q0 - prim[v][c - st], dp = prim[v][c + st] - q0;
+    b.dlt[(long long)(D * 5 + v) * N + c] = van_albada<S>(dm, dp, (T)P.lim_e2[v]);
+  }
+}
+template <typename T, bool S>
+__global__ void __launch_bounds__(256) k_slopes(DevBlock<T> b, PhysParams P) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) body_slopes<T, S, 0>(b, P, t);
+  else if (blockIdx.y == 1) body_slopes<T, S, 1>(b, P, t);
+  else body_slopes<T, S, 2>(b, P, t);
 }
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
@@ -2898,12 +2940,20 @@ __global__ void __launch_bounds__(256) k_face_split(DevBlock<T> b, PhysParams P,
   else if (blockIdx.y == 1) body_face_split<T, FAST, S, 1>(b, P, dissip_on, cd, t);
   else body_face_split<T, FAST, S, 2>(b, P, dissip_on, cd, t);
 }
-// the Roe faces (MUSCL states, upwind flux, and the viscous flux with NS)
-template <typename T>
-__global__ void __launch_bounds__(256, 3)
-    k_face_roe(const __grid_constant__ DevBlock<T> b, const __grid_constant__ PhysParams P, int dissip_on, T cd) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_ROE>(b, P, dissip_on, cd, t);
+// The Roe faces (MUSCL states, upwind flux, and the viscous flux with NS), one
+// direction per grid row.  Bound by the FP64 pipe and the latency of its chains
+// at three blocks an SM.  With the products on the integer pipes (1,300 -> 1,070
+// us a dissipative launch at 512x512x2), a direction a thread (1,058), and the states
+// and fluxes inlined instead of passed through local memory (980); two blocks
+// an SM 1,147, four 1,048.  DISS: a stage without dissipation has its own
+// instance, 379 -> 255 us at four blocks an SM.
+template <typename T, bool S, bool DISS>
+__global__ void __launch_bounds__(256, DISS ? 3 : 4)
+    k_face_roe(const __grid_constant__ DevBlock<T> b, const __grid_constant__ PhysParams P, T cd) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y == 0) body_face_split<T, false, S, 0, FACE_ROE>(b, P, DISS, cd, t);
+  else if (blockIdx.y == 1) body_face_split<T, false, S, 1, FACE_ROE>(b, P, DISS, cd, t);
+  else body_face_split<T, false, S, 2, FACE_ROE>(b, P, DISS, cd, t);
 }
 // a stage without dissipation of the central scheme: only the convective
 // face fluxes efs(q) = 0.5*(F(q) + F(q-1)), the same expression as face_dir,
@@ -3013,13 +3063,13 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
   for (int m = 1; m <= E.mstage; m++) {
     const StageArgs& A = E.st[m - 1];
     if (A.fast) {
-      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, true, false>(b, P, A.dissip_on, t);
+      for (long long t = gt; t < nprep; t += gs) body_prep<T, true, false>(b, P, A.dissip_on, t);
       g.sync();
       if (A.dissip_on)
         for (long long t = gt; t < 3 * split_row(b, 1); t += gs)
           body_face_rows<T, true, false>(b, P, 1, (T)A.cd, t);
     } else {
-      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, false, false>(b, P, A.dissip_on, t);
+      for (long long t = gt; t < nprep; t += gs) body_prep<T, false, false>(b, P, A.dissip_on, t);
       g.sync();
       for (long long t = gt; t < nface; t += gs) body_face<T, FACE_ANY, false>(b, P, A.dissip_on, (T)A.cd, t);
     }
@@ -3140,7 +3190,7 @@ template <typename T, bool FAST, bool S> struct FPrep {
   int dissip_on;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, false, FAST, S>(b, M.P[q], dissip_on, t);
+    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, FAST, S>(b, M.P[q], dissip_on, t);
   }
 };
 template <typename T, bool S> struct FFace {
@@ -3383,13 +3433,19 @@ void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, cons
     });
   } else if (part == 0) {
     long long n1 = (long long)b.ie * b.je * b.ke;
-    if (A.fast) {
-      with_form(b, [&](auto S) { k_prep<T, false, true, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on); });
-    } else if (P.distype == 2) {
-      k_prim<T><<<LAUNCH_N(b.N), 0, s>>>(b);
-      k_prep<T, true, false, true><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+    if (P.distype == 2) {
+      const auto g = rows(2);
+      with_form(b, [&](auto S) {
+        k_prim<T, S.value><<<LAUNCH_N(b.N), 0, s>>>(b, P, A.dissip_on);
+        k_slopes<T, S.value><<<g.first, g.second, 0, s>>>(b, P);
+      });
     } else {
-      with_form(b, [&](auto S) { k_prep<T, false, false, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on); });
+      with_form(b, [&](auto S) {
+        if (A.fast)
+          k_prep<T, true, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+        else
+          k_prep<T, false, S.value><<<LAUNCH_N(n1), 0, s>>>(b, P, A.dissip_on);
+      });
     }
   } else if (part == 1) {
     long long n2 = (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1);
@@ -3400,7 +3456,13 @@ void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, cons
     else if (P.distype == 0)
       k_face<T><<<LAUNCH_N(n2), 0, s>>>(b, P, A.dissip_on, (T)A.cd);
     else
-      k_face_roe<T><<<LAUNCH_N(n2), 0, s>>>(b, P, A.dissip_on, (T)A.cd);
+      with_form(b, [&](auto S) {
+        const auto g = rows(1);
+        if (A.dissip_on)
+          k_face_roe<T, S.value, true><<<g.first, g.second, 0, s>>>(b, P, (T)A.cd);
+        else
+          k_face_roe<T, S.value, false><<<g.first, g.second, 0, s>>>(b, P, (T)A.cd);
+      });
   } else if (part == 2) {
     if (b.nmir > 0) k_rec_wall<T><<<LAUNCH_N(b.nmir), 0, s>>>(b, P, A.dissip_on, (T)A.cd, err);
   } else if (part == 3) {
