@@ -31,7 +31,7 @@ struct DevBlock {
   T* qf;                    // 5N multigrid forcing
   T* vdtim;                 // N local time step
   T* lam;                   // N radi+radj+radk
-  double* dtim;             // 1 global time step (FP64 bits, atomicMin target)
+  double* dtim;             // global time step; then the blocks' running minimum and count (block_min_dtim)
   const uint8_t* blank;     // N
   const uint8_t* marker;    // N
   const int32_t* cutmap;    // N: -1 or cut-target index
@@ -57,6 +57,7 @@ struct DevBlock {
   // cut-cell records
   int nmir;
   int m0;                   // first record with an empty cloud (nmir if none)
+  int cut_beside;           // every cloud cell is physical: bc_cutcell shares the boundary launch
   const int32_t* rec_i;     // [nmir][8]: ccid(3), faceid, zz, npoint, counted in the forces, pad
   const int32_t* rec_cloud; // [nmir][8][3]
   const double* rec_coef;   // [nmir][8]
@@ -163,7 +164,8 @@ enum MultiKind {
   MK_FACE3,      // the face pass in three rows
   MK_N,          // all cells N
   MK_N5,         // 5N
-  MK_REC,        // cut-cell records
+  MK_REC,        // cut-cell records, eight lanes each
+  MK_CUT,        // the same where the solid states need a launch before the boundaries
   MK_IRS0,       // 5 * lines along i, j, k
   MK_IRS1,
   MK_IRS2,
@@ -221,7 +223,7 @@ void make_xfer_host(const int ratio[3], const int offset[3], void* out);
 template <typename T> int launch_euler_coop(const DevBlock<T>& b, const PhysParams& P, const EulerLaunch& L, int device,
                                             cudaStream_t s, bool aux32 = false);
 template <typename T> void launch_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s,
-                                           bool aux32 = false);
+                                           bool aux32 = false, bool save = false);
 template <typename T> void launch_stage(const DevBlock<T>& b, const PhysParams& P, const StageArgs& A, unsigned* err,
                                         cudaStream_t s, cudaStream_t side = nullptr, cudaEvent_t fork = nullptr,
                                         cudaEvent_t join = nullptr);
@@ -236,9 +238,10 @@ template <typename T> void launch_irs_part(int part, const DevBlock<T>& b, const
 template <typename T> void launch_solut(const DevBlock<T>& b, const PhysParams& P, double rm, double p_tot, int ns,
                                         double* out, cudaStream_t s);
 template <typename T> void launch_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s);
-// faces_only: without the edge and corner ghosts (StageArgs::faces_only)
+// faces_only: without the edge and corner ghosts (StageArgs::faces_only);
+// cut_err: with the records' solid states (blocks with cut_beside only)
 template <typename T> void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s,
-                                        bool faces_only = false);
+                                        bool faces_only = false, unsigned* cut_err = nullptr);
 // work items of the boundary launches (part 0, 1, 2; 0 items: no launch)
 template <typename T> long long bc_items(const DevBlock<T>& b, int part);
 // items of the prep (e = 2) or face (e = 1) pass in rows, and which of the two
@@ -249,7 +252,6 @@ template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& 
                                         int npartial, double* out, cudaStream_t s, unsigned* err = nullptr);
 template <typename T> void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename T> void launch_copy_ws(const DevBlock<T>& b, cudaStream_t s);
-template <typename T> void launch_save_wn(const DevBlock<T>& b, cudaStream_t s);
 template <typename T> void launch_copy_wn(const DevBlock<T>& b, cudaStream_t s);
 template <typename T> void launch_init_free(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename TC, typename TF>

@@ -142,7 +142,7 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 // --------------------------------------------------------------- timestep (timestep.f90:39-115)
 // TC is the arithmetic precision (FP64 in the plain path, FP32 in the mixed one).
-template <typename T, typename TC, bool S = true>
+template <typename T, typename TC, bool S, bool SAVE>
 __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err,
                                                             long long t) {
   const int nxl = b.nx, nyl = b.ny;
@@ -153,6 +153,10 @@ __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b
   const long long c = cidx(b.Pi, b.Pj, i, j, k);
   const TC gamma = (TC)P.gamma;
   TC w0 = (TC)b.w[c], w1 = (TC)b.w[N + c], w2 = (TC)b.w[2 * N + c], w3 = (TC)b.w[3 * N + c];
+  if (SAVE) {
+#pragma unroll
+    for (int v = 0; v < 5; v++) b.wn[v * N + c] = b.w[v * N + c];
+  }
   TC pc = (TC)b.p[c];
   TC y = pdiv<S>(TC(1), w0);
   TC cc = pmdiv<S>(pmul<S>(gamma, pc), w0, y);
@@ -226,10 +230,9 @@ __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b
   return mine;
 }
 
-// minimum over the calling block, then one atomicMin of its bits on dtim
-// (vdtim >= 0, so the IEEE bit patterns order like the values); every thread
-// of the block must call it
-__device__ __forceinline__ void block_min_to(unsigned long long mine, double* dtim) {
+// minimum over the calling block (vdtim >= 0, so the IEEE bit patterns order
+// like the values), valid in thread 0; every thread of the block must call it
+__device__ __forceinline__ unsigned long long block_min(unsigned long long mine) {
   __shared__ unsigned long long smin[32];
   for (int o = 16; o > 0; o >>= 1) {
     unsigned long long q = __shfl_down_sync(0xffffffffu, mine, o);
@@ -245,29 +248,39 @@ __device__ __forceinline__ void block_min_to(unsigned long long mine, double* dt
       unsigned long long q = __shfl_down_sync(0xffffffffu, mine, o);
       mine = q < mine ? q : mine;
     }
-    if (lane == 0 && mine != ~0ull) atomicMin((unsigned long long*)dtim, mine);
+  }
+  return mine;
+}
+// dtim = min(10, every block's minimum): the blocks meet in dtim[1] (bits) and
+// count themselves in dtim[2]; the last of nblocks writes dtim[0] and leaves the
+// other two as it found them (~0 and 0), so no launch has to reset them
+__device__ __forceinline__ void block_min_dtim(unsigned long long mine, double* dtim, int nblocks) {
+  mine = block_min(mine);
+  if (threadIdx.x != 0) return;
+  unsigned long long* run = (unsigned long long*)(dtim + 1);
+  unsigned* count = (unsigned*)(dtim + 2);
+  if (mine != ~0ull) atomicMin(run, mine);
+  __threadfence();
+  if (atomicAdd(count, 1u) == (unsigned)nblocks - 1) {
+    __threadfence();
+    const unsigned long long m = atomicExch(run, ~0ull), ten = (unsigned long long)__double_as_longlong(10.0);
+    *count = 0u;
+    *dtim = __longlong_as_double((long long)(m < ten ? m : ten));
   }
 }
 
-template <typename T, typename TC, bool S>
+// SAVE: wn = w as well (euler.f90:80-83), from the values the cell has loaded
+template <typename T, typename TC, bool S, bool SAVE>
 __global__ void k_timestep(DevBlock<T> b, PhysParams P, unsigned* err) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long mine = ~0ull;
-  if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC, S>(b, P, err, t);
-  block_min_to(mine, b.dtim);  // global dtim (timestep.f90:112), kept even when vt = 0
+  if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC, S, SAVE>(b, P, err, t);
+  block_min_dtim(mine, b.dtim, gridDim.x);  // global dtim (timestep.f90:112), kept even when vt = 0
 }
 
 template <typename T> __global__ void k_set_scalar(T* p, double v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *p = (T)v;
 }
-// dtim travels as the bit pattern of a double (atomicMin on positive doubles)
-__global__ void k_dtim_reset(double* p) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *p = 10.0;
-}
-template <typename T> __global__ void k_dtim_convert(double* src, T* dst) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *dst = (T)(*src);
-}
-
 // --------------------------------------------------------------- stage: per-cell pass
 // Box [1..ie]x[1..je]x[1..ke]: every cell whose flux or sensor a face needs.
 template <bool S, typename T>
@@ -1114,6 +1127,108 @@ __global__ void k_rec_wall(const __grid_constant__ DevBlock<T> b, const __grid_c
   if (m < b.nmir) rec_wall_terms(b, P, dissip_on, cd, err, m);
 }
 
+__host__ __device__ __forceinline__ int pad32(int n) { return (n + 31) & ~31; }
+template <typename T> __host__ __device__ __forceinline__ int rec_lane_items(const DevBlock<T>& b) {
+  return pad32(8 * b.nmir);
+}
+// the scheme of the split passes and of rec_wall_lanes
+__host__ __device__ __forceinline__ bool split_scheme(const PhysParams& P) {
+  return P.distype == 0 && !P.eqn_ns && !P.matrix;
+}
+
+// rec_wall_terms for the central scheme with scalar dissipation of the Euler
+// equations, eight lanes a record: lane v < 5 forms variable v, and the six
+// divisions (three sensors, three reciprocals of densities) go to six lanes.
+// One thread a record ran 3,000 instructions in a row, 20 us by events on any
+// level; this takes 9.  Same operations, same order, same bits.  Every lane of
+// a warp calls it.
+template <typename T>
+__device__ __forceinline__ void rec_wall_lanes(const DevBlock<T>& b, const PhysParams& P, int dissip_on, T cd,
+                                               unsigned* err, int t) {
+  const int lane = t & 7;
+  const bool own = (t >> 3) < b.nmir;
+  const int m = own ? t >> 3 : b.nmir - 1;
+  const int v = lane < 5 ? lane : 4;
+  const long long N = b.N;
+  const int* ri = b.rec_i + 8 * m;
+  const int D = ri[4] - 1;
+  const long long st = D == 0 ? 1 : (D == 1 ? (long long)b.Pi : (long long)b.Pi * b.Pj);
+  const long long c = cidx(b.Pi, b.Pj, ri[0], ri[1], ri[2]);
+  const bool plus = ri[3] >= 4;  // solid on the + side
+  const int es = plus ? -1 : 1;  // along the axis, away from the wall
+  const long long e = es * st;
+  const T s = D == 0 ? (T)b.s[0] : (D == 1 ? (T)b.s[1] : (T)b.s[2]);
+  const int pos = D == 0 ? ri[0] : (D == 1 ? ri[1] : ri[2]);
+  const int lim = D == 0 ? b.ib : (D == 1 ? b.jb : b.kb);
+  const bool third = plus ? pos - 3 >= 0 : pos + 3 <= lim;
+  const T* wv = b.w + v * N + c;
+  const T w0 = wv[0], w1 = wv[e], w2 = wv[2 * e], ws = b.rec_wsol[5 * m + v], psol = b.rec_psol[m];
+  const T p0 = b.p[c], p1 = b.p[c + e], p2 = b.p[c + 2 * e], p3 = third ? b.p[c + 3 * e] : T(0);
+  const int lq = D == 0 ? b.il : (D == 1 ? b.jl : b.kl);
+  const int q1 = pos + es < 2 ? 2 : (pos + es > lq ? lq : pos + es);  // the ghost-copy rule of timestep.f90:227-282
+  const T lam0 = b.lam[c], lam1 = b.lam[c + (long long)(q1 - pos) * st];
+  auto from = [&](T x, int l) { return __shfl_sync(0xffffffffu, x, l, 8); };
+  // a division a lane: the sensors beside the wall, one cell on and two cells
+  // on, in the argument order of dfluxb.f90's three axes; then 1/rho at the
+  // cut cell, the solid state and the neighbour
+  const bool fwd = plus && D != 0;
+  const T r0 = from(w0, 0), rs = from(ws, 0), r1 = from(w1, 0);
+  T num = T(1), den = lane == 3 ? r0 : (lane == 4 ? rs : r1);
+  if (lane < 3) {
+    const T x = lane == 0 ? (fwd ? psol : p1) : (lane == 1 ? (fwd ? p0 : p2) : (plus ? p1 : p3));
+    const T y = lane == 0 ? p0 : (lane == 1 ? p1 : p2);
+    const T z = lane == 0 ? (fwd ? p1 : psol) : (lane == 1 ? (fwd ? p2 : p0) : (plus ? p3 : p1));
+    num = fabs(x - T(2) * y + z);
+    den = fabs(x + T(2) * y + z);
+  }
+  const T quot = num / den;
+  const T s0 = from(quot, 0), s1 = from(quot, 1), sq = from(quot, 2), s2 = third ? sq : T(0);
+  const T y0 = from(quot, 3), ys = from(quot, 4), y1 = from(quot, 5);
+  // ceflux of the three states (efluxb.f90:66-110)
+  auto flux = [&](T x, T p, T rho, T y) -> T {
+    const T f0 = from(x, 1 + D) * s;
+    const T q = lane == 4 ? f0 * (x + p) : f0 * x;
+    T f = lane == 0 ? f0 : mdiv(q, rho, y);
+    if (lane == 1 + D) f = f + p * s;
+    return f;
+  };
+  const T f1 = flux(w0, p0, r0, y0), f2 = flux(ws, psol, rs, ys), f3 = flux(w1, p1, r1, y1);
+  const T fs = T(0.5) * (f1 + f2), fa = T(0.5) * (f1 + f3);
+  T* W = b.rec_wall + 25LL * m;
+  const bool put = own && lane < 5;
+  if (put) {
+    W[v] = plus ? fa : fs;
+    W[5 + v] = plus ? fs : fa;
+  }
+  if (own && lane == 0 && fabs(w0) < T(1.0e-8)) atomicCAS(err, 0u, (unsigned)ERR_ZERORHO);
+  if (!dissip_on) return;
+  // dfluxb.f90:29-423; the fifth variable is the enthalpy
+  const T W0 = lane == 4 ? w0 + p0 : w0, W1 = lane == 4 ? w1 + p1 : w1, W2 = lane == 4 ? w2 + p2 : w2;
+  const T Ws = lane == 4 ? ws + psol : ws;
+  const T A = plus ? s1 : s0, B = plus ? s0 : s1;
+  const T near = fmaxT(A, B);
+  auto face = [&](T ep, T lam, T x2, T x1, T x0) -> T {
+    T dis2 = (T)P.vis2 * ep;
+    T dis4 = fdimT((T)P.vis4, dis2);
+    dis2 = dis2 * cd;
+    dis4 = dis4 * cd;
+    const T f = x2 - T(2) * x1 + x0;
+    return (dis2 * x1 - dis4 * f) * lam;
+  };
+  const T dw = plus ? Ws - W0 : W0 - Ws, d1 = plus ? W0 - W1 : W1 - W0, d2 = plus ? W1 - W2 : W2 - W1;
+  const T wall = face(near, lam0, plus ? dw : d1, dw, plus ? d1 : dw);
+  const T next = face(fmaxT(near, s2), T(0.5) * (plus ? lam1 + lam0 : lam0 + lam1), plus ? dw : d2, d1, plus ? d2 : dw);
+  if (put) {
+    W[15 + v] = plus ? next - wall : wall - next;
+    W[20 + v] = next;
+  }
+}
+template <typename T>
+__global__ void k_rec_lanes(DevBlock<T> b, PhysParams P, int dissip_on, T cd, unsigned* err) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < rec_lane_items(b)) rec_wall_lanes(b, P, dissip_on, cd, err, t);
+}
+
 // the record's geometry: cell, axis stride, solid side
 template <typename T>
 __device__ __forceinline__ void rec_geom(const DevBlock<T>& b, int m, long long& c, long long& st, int& D, bool& plus) {
@@ -1285,7 +1400,7 @@ __device__ __forceinline__ void body_combine(const DevBlock<T>& b, const PhysPar
       }
     }
   }
-  if (A.dissip_on || A.scale_fw) {
+  if (A.dissip_on || A.scale_fw || A.m == 1) {  // the first stage starts fw
 #pragma unroll
     for (int v = 0; v < 5; v++) b.fw[v * N + c] = fwv[v];
   }
@@ -1919,53 +2034,65 @@ __device__ __forceinline__ void body_update(const DevBlock<T>& b, const PhysPara
 }
 
 // --------------------------------------------------------------- bc_cutcell (bc_cutcell.f90:40-268)
+// Eight lanes a record: lane q fetches cloud cell q's place and weight, lane v
+// sums variable v over the cloud (lane 5 the pressure) in the cloud's order with
+// its eight loads in flight together, and lanes 0-2 divide the normal's
+// components.  One thread a record walked the cloud 48 loads in a row, 20-34 us
+// by events; this takes 10 by itself and nothing beside the face ghosts.  Every
+// lane of a warp calls it.
 template <typename T>
-__device__ void body_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned* err, int m) {
-  if (m >= b.nmir || m > b.m0) return;
+__device__ __forceinline__ void cutcell_lanes(const DevBlock<T>& b, const PhysParams& P, unsigned* err, int t) {
+  const int lane = t & 7, v = lane < 5 ? lane : 0;
+  const int mm = t >> 3, m = mm < b.nmir ? mm : b.nmir - 1;
+  const bool own = mm < b.nmir && mm <= b.m0;  // after the first empty cloud the reference returns
+  const bool empty = m == b.m0;
   T* ws = b.rec_wsol + 5LL * m;
-  if (m == b.m0) {  // empty cloud: zero this record; the reference returns here
-    for (int v = 0; v < 5; v++) ws[v] = T(0);
-    b.rec_psol[m] = T(0);
-    return;
-  }
   const long long N = b.N;
   const int ncl = b.rec_i[8 * m + 5];
+  auto from = [&](T x, int l) { return __shfl_sync(0xffffffffu, x, l, 8); };
+  const int* ijk = b.rec_cloud + (8 * m + (lane < ncl ? lane : 0)) * 3;
+  const int cl = (int)cidx(b.Pi, b.Pj, ijk[0], ijk[1], ijk[2]);
+  const T cf = (T)b.rec_coef[8 * m + lane];
+  const T* src = lane == 5 ? b.p : b.w + v * N;
+  T x[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) x[q] = src[__shfl_sync(0xffffffffu, cl, q, 8)];
+  T sum = T(0);
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const T a = from(cf, q);
+    if (q < ncl) sum = sum + a * x[q];
+  }
   T nv[3] = {(T)b.rec_nvec[3 * m], (T)b.rec_nvec[3 * m + 1], (T)b.rec_nvec[3 * m + 2]};
-  T qb[3] = {(T)b.rec_qb[3 * m], (T)b.rec_qb[3 * m + 1], (T)b.rec_qb[3 * m + 2]};
-  T nn = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
-  for (int q = 0; q < 3; q++) nv[q] = nv[q] / nn;
-  long long cl[8];
-  T cf[8];
-  for (int q = 0; q < ncl; q++) {
-    const int* ijk = b.rec_cloud + (8 * m + q) * 3;
-    cl[q] = cidx(b.Pi, b.Pj, ijk[0], ijk[1], ijk[2]);
-    cf[q] = (T)b.rec_coef[8 * m + q];
-  }
-  T vr[5];
-  for (int v = 0; v < 5; v++) {
-    T a = T(0);
-    for (int q = 0; q < ncl; q++) a = a + cf[q] * b.w[v * N + cl[q]];
-    vr[v] = a;
-  }
-  T pr = T(0);
-  for (int q = 0; q < ncl; q++) pr = pr + cf[q] * b.p[cl[q]];
-  T wsol[5], psol = pr;
-  const T gm1 = (T)P.gamma - T(1);
+  const T qb[3] = {(T)b.rec_qb[3 * m], (T)b.rec_qb[3 * m + 1], (T)b.rec_qb[3 * m + 2]};
+  const T nn = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
+  const T nq = (lane == 0 ? nv[0] : (lane == 1 ? nv[1] : nv[2])) / nn;
+#pragma unroll
+  for (int q = 0; q < 3; q++) nv[q] = from(nq, q);
+  T wsol[5];
+#pragma unroll
+  for (int q = 0; q < 5; q++) wsol[q] = from(sum, q);
+  const T psol = from(sum, 5);
   if (!P.eqn_ns) {
-    for (int v = 0; v < 5; v++) wsol[v] = vr[v];
-    T qn = T(2) * (nv[0] * (wsol[1] - wsol[0] * qb[0]) + nv[1] * (wsol[2] - wsol[0] * qb[1]) +
-                   nv[2] * (wsol[3] - wsol[0] * qb[2]));
+    const T qn = T(2) * (nv[0] * (wsol[1] - wsol[0] * qb[0]) + nv[1] * (wsol[2] - wsol[0] * qb[1]) +
+                         nv[2] * (wsol[3] - wsol[0] * qb[2]));
+#pragma unroll
     for (int q = 0; q < 3; q++) wsol[1 + q] = wsol[1 + q] - qn * nv[q];
   } else {
-    wsol[0] = vr[0];
-    for (int q = 0; q < 3; q++) wsol[1 + q] = T(2) * qb[q] * vr[0] - vr[1 + q];
+#pragma unroll
+    for (int q = 0; q < 3; q++) wsol[1 + q] = T(2) * qb[q] * wsol[0] - wsol[1 + q];
   }
-  wsol[4] = psol / gm1 + T(0.5) * (wsol[1] * wsol[1] + wsol[2] * wsol[2] + wsol[3] * wsol[3]) / wsol[0];
+  wsol[4] = psol / ((T)P.gamma - T(1)) +
+            T(0.5) * (wsol[1] * wsol[1] + wsol[2] * wsol[2] + wsol[3] * wsol[3]) / wsol[0];
   bool nan = false;
-  for (int v = 0; v < 5; v++) nan |= (wsol[v] != wsol[v]);
-  if (nan && !P.eqn_ns) atomicCAS(err, 0u, (unsigned)ERR_NAN);
-  for (int v = 0; v < 5; v++) ws[v] = wsol[v];
-  b.rec_psol[m] = psol;
+#pragma unroll
+  for (int q = 0; q < 5; q++) nan |= (wsol[q] != wsol[q]);
+  if (!own) return;
+  if (nan && !empty && !P.eqn_ns && lane == 0) atomicCAS(err, 0u, (unsigned)ERR_NAN);
+  // an empty cloud: this record is zeroed
+  const T r = lane == 0 ? wsol[0] : (lane == 1 ? wsol[1] : (lane == 2 ? wsol[2] : (lane == 3 ? wsol[3] : wsol[4])));
+  if (lane < 5) ws[lane] = empty ? T(0) : r;
+  if (lane == 5) b.rec_psol[m] = empty ? T(0) : psol;
 }
 
 // --------------------------------------------------------------- face boundary conditions
@@ -2155,7 +2282,6 @@ template <typename T>
 __host__ __device__ __forceinline__ bool bc_whole(const DevBlock<T>& b) {
   return b.bctype[0] && b.bctype[1] && b.bctype[2] && b.bctype[3] && b.bctype[4] && b.bctype[5];
 }
-__host__ __device__ __forceinline__ int pad32(int n) { return (n + 31) & ~31; }
 // work items, in whole warps: the face ghosts (an item writes both layers);
 // the ghost cells with two or three ghost axes (without the corner cells when
 // those share the launch); the corner cells, four lanes each
@@ -2172,7 +2298,7 @@ __host__ __device__ __forceinline__ int bc_n3(const DevBlock<T>& b) {
   return pad32(4 * (4 * b.nz + 4 * b.ny + 4 * (b.nx + 2) + 8));
 }
 template <typename T> long long bc_items_t(const DevBlock<T>& b, int part) {
-  if (part == 0) return bc_n1(b);
+  if (part == 0) return (long long)bc_n1(b) + (b.cut_beside ? rec_lane_items(b) : 0);
   if (part == 1) return (long long)bc_n2(b) + (bc_whole(b) ? bc_n3(b) : 0);
   return bc_whole(b) ? 0 : bc_n3(b);
 }
@@ -2349,12 +2475,19 @@ __device__ __forceinline__ void body_bc_corner(const DevBlock<T>& b, const PhysP
   store_cell(b, cidx(b.Pi, b.Pj, i, j, k), o);
 }
 
-// part 0: the face ghosts; 1: the edge and corner ghosts; 2: the corner cells
-// of blocks with a face without a boundary condition
+// part 0: the face ghosts and, with cut, the records' solid states where every
+// cloud cell is physical (bc_cutcell then reads none of the ghosts and writes
+// only the records); 1: the edge and corner ghosts; 2: the corner cells of
+// blocks with a face without a boundary condition
 template <typename T, int PART>
-__device__ __forceinline__ void body_bcond(const DevBlock<T>& b, const PhysParams& P, long long t) {
+__device__ __forceinline__ void body_bcond(const DevBlock<T>& b, const PhysParams& P, unsigned* err, int cut,
+                                           long long t) {
   if (PART == 0) {
-    if (t < bc_n1(b)) body_bc_face(b, P, (int)t);
+    const int n1 = bc_n1(b);
+    if (t < n1)
+      body_bc_face(b, P, (int)t);
+    else if (cut && b.cut_beside && t < (long long)n1 + rec_lane_items(b))
+      cutcell_lanes(b, P, err, (int)t - n1);
   } else if (PART == 1) {
     const int n2 = bc_n2(b);
     if (t < n2)
@@ -2365,9 +2498,14 @@ __device__ __forceinline__ void body_bcond(const DevBlock<T>& b, const PhysParam
     if (!bc_whole(b) && t < bc_n3(b)) body_bc_corner(b, P, (int)t);
   }
 }
+// Bound by latency at every size that matters: a far-field ghost is a chain
+// of some 1,100 dependent instructions.  Three launches for the faces and
+// three for the corners, each item of a warp on a branch of its own, took 74 us
+// a stage on a 24^3 block; these take 9 us for the faces and, after the last
+// stage of an inviscid update only (StageArgs::faces_only), 15 us more.
 template <typename T, int PART>
-__global__ void k_bcond(DevBlock<T> b, PhysParams P) {
-  body_bcond<T, PART>(b, P, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void k_bcond(DevBlock<T> b, PhysParams P, unsigned* err, int cut) {
+  body_bcond<T, PART>(b, P, err, cut, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // --------------------------------------------------------------- residual norm (euler.f90:431-447)
@@ -2452,27 +2590,10 @@ __global__ void k_copy5(const T* __restrict__ src, T* __restrict__ dst, long lon
   if (c < n) dst[c] = src[c];
 }
 
-// wn = w on physical cells, dw = fw = 0 everywhere (euler.f90:80-89)
-template <typename T>
-__device__ __forceinline__ void body_save_wn(const DevBlock<T>& b, long long c) {
-  const long long N = b.N;
-  int i, j, k;
-  cell_of(c, b.Pi, b.Pj, 0, i, j, k);
-  bool phys = i >= 2 && i <= b.il && j >= 2 && j <= b.jl && k >= 2 && k <= b.kl;
-  for (int v = 0; v < 5; v++) {
-    if (phys) b.wn[v * N + c] = b.w[v * N + c];
-    b.dw[v * N + c] = T(0);
-    b.fw[v * N + c] = T(0);
-  }
-}
-
-template <typename T>
-__global__ void k_save_wn(DevBlock<T> b) {
-  long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < b.N) body_save_wn(b, c);
-}
-
-// wn = w on physical cells only (movco.f90:29-35)
+// wn = w on physical cells (euler.f90:80-83, movco.f90:29-35).  The zeros
+// euler.f90:84-89 puts into dw and fw need no pass: a stage writes dw whole before
+// anything reads it, the first stage writes fw, and no ghost of either is
+// ever written after the zeros of their allocation.
 template <typename T>
 __device__ __forceinline__ void body_copy_wn(const DevBlock<T>& b, long long c) {
   if (c >= b.N) return;
@@ -2997,8 +3118,8 @@ __global__ void k_update(DevBlock<T> b, PhysParams P, StageArgs A) {
 }
 template <typename T>
 __global__ void k_cutcell(DevBlock<T> b, PhysParams P, unsigned* err) {
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  body_cutcell(b, P, err, m);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < rec_lane_items(b)) cutcell_lanes(b, P, err, t);
 }
 // =============================================================== one euler update in one launch
 // For the small coarse grids of the multigrid hierarchy every phase of
@@ -3044,19 +3165,19 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
   const long long gs = (long long)gridDim.x * blockDim.x;
   const long long ncell = (long long)b.nx * b.ny * b.nz;
   if (E.do_timestep) {
-    if (gt == 0) *b.dtim = 10.0;
-    g.sync();
+    const int nb = (int)((ncell + blockDim.x - 1) / blockDim.x);
     for (long long base = (long long)blockIdx.x * blockDim.x; base < ncell; base += gs) {
       long long t = base + threadIdx.x;
       unsigned long long mine = ~0ull;
-      if (t < ncell) mine = body_timestep<T, TA, false>(b, P, E.err, t);
-      block_min_to(mine, b.dtim);
+      if (t < ncell) mine = body_timestep<T, TA, false, true>(b, P, E.err, t);
+      block_min_dtim(mine, b.dtim, nb);
     }
     g.sync();
   }
   if (E.lfir)
     for (long long q = gt; q < 5 * b.N; q += gs) b.ws[q] = b.w[q];
-  for (long long q = gt; q < b.N; q += gs) body_save_wn(b, q);
+  if (!E.do_timestep)
+    for (long long q = gt; q < b.N; q += gs) body_copy_wn(b, q);
   g.sync();
   const long long nprep = (long long)b.ie * b.je * b.ke;
   const long long nface = (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1);
@@ -3073,7 +3194,12 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
       g.sync();
       for (long long t = gt; t < nface; t += gs) body_face<T, FACE_ANY, false>(b, P, A.dissip_on, (T)A.cd, t);
     }
-    for (long long t = gt; t < b.nmir; t += gs) rec_wall_terms(b, P, A.dissip_on, (T)A.cd, E.err, (int)t);
+    if (split_scheme(P)) {
+      const long long lt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+      for (long long t = lt; t < rec_lane_items(b); t += gs) rec_wall_lanes(b, P, A.dissip_on, (T)A.cd, E.err, (int)t);
+    } else {
+      for (long long t = gt; t < b.nmir; t += gs) rec_wall_terms(b, P, A.dissip_on, (T)A.cd, E.err, (int)t);
+    }
     g.sync();
     if (A.fast)
       for (long long t = gt; t < ncell; t += gs) body_combine<T, true, false>(b, P, A, E.err, t);
@@ -3101,17 +3227,19 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
       for (long long t = gt; t < ncell; t += gs) body_update<T, false>(b, P, A, t);
       g.sync();
     }
-    for (long long t = gt; t < b.nmir; t += gs) body_cutcell(b, P, E.err, (int)t);
-    g.sync();
-    // whole warps of consecutive items: the corner cells share lanes
+    // whole warps of consecutive items: the corner cells and records share lanes
     const long long lt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (long long t = lt; t < bc_n1(b); t += gs) body_bcond<T, 0>(b, P, t);
+    if (!b.cut_beside && b.nmir > 0) {
+      for (long long t = lt; t < rec_lane_items(b); t += gs) cutcell_lanes(b, P, E.err, (int)t);
+      g.sync();
+    }
+    for (long long t = lt; t < bc_n1(b) + rec_lane_items(b); t += gs) body_bcond<T, 0>(b, P, E.err, 1, t);
     g.sync();
     if (m < E.mstage && A.faces_only) continue;
-    for (long long t = lt; t < bc_n2(b) + (bc_whole(b) ? bc_n3(b) : 0); t += gs) body_bcond<T, 1>(b, P, t);
+    for (long long t = lt; t < bc_n2(b) + (bc_whole(b) ? bc_n3(b) : 0); t += gs) body_bcond<T, 1>(b, P, E.err, 0, t);
     g.sync();
     if (!bc_whole(b)) {
-      for (long long t = lt; t < bc_n3(b); t += gs) body_bcond<T, 2>(b, P, t);
+      for (long long t = lt; t < bc_n3(b); t += gs) body_bcond<T, 2>(b, P, E.err, 0, t);
       g.sync();
     }
   }
@@ -3162,28 +3290,19 @@ __global__ void __launch_bounds__(256) k_multi(MultiArgs<T> M, F f) {
   f(M, q, base - M.off[q] + threadIdx.x);
 }
 
-template <typename T> struct FDtimReset {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t == 0) *M.B[q].dtim = 10.0;
-  }
-};
 template <typename T, typename TC, bool S> struct FTimestep {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
     unsigned long long mine = ~0ull;
-    if (t < (long long)b.nx * b.ny * b.nz) mine = body_timestep<T, TC, S>(b, M.P[q], M.err[q], t);
-    block_min_to(mine, b.dtim);
+    const long long n = (long long)b.nx * b.ny * b.nz;
+    if (t < n) mine = body_timestep<T, TC, S, true>(b, M.P[q], M.err[q], t);
+    block_min_dtim(mine, b.dtim, (int)((n + 255) / 256));  // a call per 256 cells, whichever block makes it
   }
 };
 template <typename T> struct FCopyWs {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
     const DevBlock<T>& b = M.B[q];
     if (t < 5 * b.N) b.ws[t] = b.w[t];
-  }
-};
-template <typename T> struct FSaveWn {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t < M.B[q].N) body_save_wn(M.B[q], t);
   }
 };
 template <typename T, bool FAST, bool S> struct FPrep {
@@ -3221,7 +3340,11 @@ template <typename T> struct FRec {
   int dissip_on;
   T cd;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t < M.B[q].nmir) rec_wall_terms(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
+    if (split_scheme(M.P[q])) {
+      if (t < rec_lane_items(M.B[q])) rec_wall_lanes(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
+    } else if (t < M.B[q].nmir) {
+      rec_wall_terms(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
+    }
   }
 };
 template <typename T, bool FAST, bool S> struct FCombine {
@@ -3264,12 +3387,14 @@ template <typename T, bool S> struct FUpdate {
 };
 template <typename T> struct FCutcell {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (t < M.B[q].nmir) body_cutcell(M.B[q], M.P[q], M.err[q], (int)t);
+    // the blocks whose records do not share the boundary launch
+    if (!M.B[q].cut_beside && t < rec_lane_items(M.B[q])) cutcell_lanes(M.B[q], M.P[q], M.err[q], (int)t);
   }
 };
 template <typename T, int PART> struct FBcond {
+  int cut;
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    body_bcond<T, PART>(M.B[q], M.P[q], t);
+    body_bcond<T, PART>(M.B[q], M.P[q], M.err[q], cut, t);
   }
 };
 template <typename T> struct FDepvars {
@@ -3381,7 +3506,6 @@ template <typename T, typename F> void with_form(const DevBlock<T>& b, F&& f) {
 // 120 but face 134 against 124; 192^3 face 962 against 897.  The contracted
 // dissipation faces share nothing between the directions, and split they keep
 // twice the warps resident: 414 against 563 us a launch at 192^3.
-inline bool split_scheme(const PhysParams& P) { return P.distype == 0 && !P.eqn_ns && !P.matrix; }
 inline bool split_prep(bool fast, long long cells) { return cells <= (fast ? 300000 : 1000000); }
 inline bool split_face(bool fast, long long cells) { return fast || cells <= 300000; }
 
@@ -3394,14 +3518,20 @@ void launch_solut(const DevBlock<T>& b, const PhysParams& P, double rm, double p
 
 
 template <typename T>
-void launch_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s, bool aux32) {
+void launch_timestep(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s, bool aux32, bool save) {
   long long n = (long long)b.nx * b.ny * b.nz;
-  k_dtim_reset<<<1, 32, 0, s>>>(b.dtim);
   with_form(b, [&](auto S) {
+    auto go = [&](auto tc, auto form) {
+      using TC = decltype(tc);
+      if (save)
+        k_timestep<T, TC, form.value, true><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+      else
+        k_timestep<T, TC, form.value, false><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+    };
     if (aux32)
-      k_timestep<T, float, true><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+      go(float(), std::true_type{});
     else
-      k_timestep<T, T, S.value><<<LAUNCH_N(n), 0, s>>>(b, P, err);
+      go(T(), S);
   });
 }
 
@@ -3464,7 +3594,10 @@ void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, cons
           k_face_roe<T, S.value, false><<<g.first, g.second, 0, s>>>(b, P, (T)A.cd);
       });
   } else if (part == 2) {
-    if (b.nmir > 0) k_rec_wall<T><<<LAUNCH_N(b.nmir), 0, s>>>(b, P, A.dissip_on, (T)A.cd, err);
+    if (b.nmir > 0 && split_scheme(P))
+      k_rec_lanes<T><<<LAUNCH_N(rec_lane_items(b)), 0, s>>>(b, P, A.dissip_on, (T)A.cd, err);
+    else if (b.nmir > 0)
+      k_rec_wall<T><<<LAUNCH_N(b.nmir), 0, s>>>(b, P, A.dissip_on, (T)A.cd, err);
   } else if (part == 3) {
     long long n3 = (long long)b.nx * b.ny * b.nz;
     with_form(b, [&](auto S) {
@@ -3477,23 +3610,24 @@ void launch_stage_part(int part, const DevBlock<T>& b, const PhysParams& P, cons
 }
 
 // One stage.  With a side stream and two events, the record pass runs on the
-// side stream beside the face pass (it needs only the prep pass's output);
-// the combine pass waits for both.
+// side stream beside the prep and face passes (it needs only the state); the
+// combine pass waits for both.
 template <typename T>
 void launch_stage(const DevBlock<T>& b, const PhysParams& P, const StageArgs& A, unsigned* err, cudaStream_t s,
                   cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
-  launch_stage_part<T>(0, b, P, A, err, s);
   const bool beside = b.nmir > 0 && side && fork && join;
   if (beside) {
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
     launch_stage_part<T>(2, b, P, A, err, side);
     cudaEventRecord(join, side);
-  } else {
-    launch_stage_part<T>(2, b, P, A, err, s);
   }
+  launch_stage_part<T>(0, b, P, A, err, s);
   launch_stage_part<T>(1, b, P, A, err, s);
-  if (beside) cudaStreamWaitEvent(s, join, 0);
+  if (beside)
+    cudaStreamWaitEvent(s, join, 0);
+  else
+    launch_stage_part<T>(2, b, P, A, err, s);
   launch_stage_part<T>(3, b, P, A, err, s);
 }
 
@@ -3616,16 +3750,16 @@ void launch_irs(const DevBlock<T>& b, const PhysParams& P, const IrsTables* tab,
 
 template <typename T>
 void launch_cutcell(const DevBlock<T>& b, const PhysParams& P, unsigned* err, cudaStream_t s) {
-  if (b.nmir > 0) k_cutcell<T><<<LAUNCH_N(b.nmir), 0, s>>>(b, P, err);
+  if (b.nmir > 0) k_cutcell<T><<<LAUNCH_N(rec_lane_items(b)), 0, s>>>(b, P, err);
 }
 
 template <typename T>
-void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s, bool faces_only) {
-  k_bcond<T, 0><<<LAUNCH_N(bc_items_t(b, 0)), 0, s>>>(b, P);
+void launch_bcond(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s, bool faces_only, unsigned* cut_err) {
+  k_bcond<T, 0><<<LAUNCH_N(cut_err ? bc_items_t(b, 0) : bc_n1(b)), 0, s>>>(b, P, cut_err, cut_err != nullptr);
   if (faces_only) return;
-  k_bcond<T, 1><<<LAUNCH_N(bc_items_t(b, 1)), 0, s>>>(b, P);
+  k_bcond<T, 1><<<LAUNCH_N(bc_items_t(b, 1)), 0, s>>>(b, P, nullptr, 0);
   const long long n = bc_items_t(b, 2);
-  if (n > 0) k_bcond<T, 2><<<LAUNCH_N(n), 0, s>>>(b, P);
+  if (n > 0) k_bcond<T, 2><<<LAUNCH_N(n), 0, s>>>(b, P, nullptr, 0);
 }
 
 template <typename T>
@@ -3750,11 +3884,6 @@ void launch_copy_ws(const DevBlock<T>& b, cudaStream_t s) {
 }
 
 template <typename T>
-void launch_save_wn(const DevBlock<T>& b, cudaStream_t s) {
-  k_save_wn<T><<<nblk(b.N, TPB), TPB, 0, s>>>(b);
-}
-
-template <typename T>
 void launch_copy_wn(const DevBlock<T>& b, cudaStream_t s) {
   k_copy_wn<T><<<nblk(b.N, TPB), TPB, 0, s>>>(b);
 }
@@ -3834,11 +3963,11 @@ static MultiArgs<T> multi_args(const MultiLevel& L) {
 }
 
 template <typename T>
-static void multi_bcond(const MultiLevel& L, MultiArgs<T>& M, cudaStream_t s, bool faces_only = false) {
-  go_multi(L, M, MK_BC0, FBcond<T, 0>{}, s);
+static void multi_bcond(const MultiLevel& L, MultiArgs<T>& M, cudaStream_t s, bool faces_only = false, int cut = 0) {
+  go_multi(L, M, MK_BC0, FBcond<T, 0>{cut}, s);
   if (faces_only) return;
-  go_multi(L, M, MK_BC1, FBcond<T, 1>{}, s);
-  go_multi(L, M, MK_BC2, FBcond<T, 2>{}, s);
+  go_multi(L, M, MK_BC1, FBcond<T, 1>{0}, s);
+  go_multi(L, M, MK_BC2, FBcond<T, 2>{0}, s);
 }
 
 // timestep (optionally) and euler.f90:1-462 on one block of every case: the
@@ -3848,14 +3977,13 @@ static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, b
                           bool rt, cudaStream_t s) {
   MultiArgs<T> M = multi_args<T>(L);
   if (with_timestep) {
-    go_multi(L, M, MK_ONE, FDtimReset<T>{}, s);
     if (L.aux32)
       go_multi(L, M, MK_PHYS, FTimestep<T, float, true>{}, s);
     else
       go_multi(L, M, MK_PHYS, FTimestep<T, T, S>{}, s);
   }
   if (lfir) go_multi(L, M, MK_N5, FCopyWs<T>{}, s);
-  go_multi(L, M, MK_N, FSaveWn<T>{}, s);
+  if (!with_timestep) go_multi(L, M, MK_N, FCopyWn<T>{}, s);
   for (int m = 1; m <= mstage; m++) {
     const StageArgs& a = A[m - 1];
     if (L.prep_rows && L.fast)
@@ -3899,8 +4027,8 @@ static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, b
       }
       go_multi(L, M, MK_PHYS, FUpdate<T, S>{a}, s);
     }
-    go_multi(L, M, MK_REC, FCutcell<T>{}, s);
-    multi_bcond(L, M, s, a.faces_only && m < mstage);
+    go_multi(L, M, MK_CUT, FCutcell<T>{}, s);
+    multi_bcond(L, M, s, a.faces_only && m < mstage, 1);
   }
   if (rt) {
     go_multi(L, M, MK_RTP, FRtrmsPartial<T>{}, s);
@@ -3965,12 +4093,10 @@ template <typename T, typename TA>
 __global__ void __launch_bounds__(256, 1) k_group_euler(MultiArgs<T> M, GroupEuler G) {
   cg::grid_group grid = cg::this_grid();
   if (G.do_timestep) {
-    group_phase(M, G, MK_ONE, FDtimReset<T>{});
-    grid.sync();
     group_phase(M, G, MK_PHYS, FTimestep<T, TA, false>{});
   }
   if (G.lfir) group_phase(M, G, MK_N5, FCopyWs<T>{});
-  group_phase(M, G, MK_N, FSaveWn<T>{});
+  if (!G.do_timestep) group_phase(M, G, MK_N, FCopyWn<T>{});
   grid.sync();
   for (int m = 1; m <= G.mstage; m++) {
     const StageArgs& a = G.st[m - 1];
@@ -4016,15 +4142,17 @@ __global__ void __launch_bounds__(256, 1) k_group_euler(MultiArgs<T> M, GroupEul
       group_phase(M, G, MK_PHYS, FUpdate<T, false>{a});
       grid.sync();
     }
-    group_phase(M, G, MK_REC, FCutcell<T>{});
-    grid.sync();
-    group_phase(M, G, MK_BC0, FBcond<T, 0>{});
+    if (G.tot[MK_CUT] > 0) {
+      group_phase(M, G, MK_CUT, FCutcell<T>{});
+      grid.sync();
+    }
+    group_phase(M, G, MK_BC0, FBcond<T, 0>{1});
     grid.sync();
     if (a.faces_only && m < G.mstage) continue;
-    group_phase(M, G, MK_BC1, FBcond<T, 1>{});
+    group_phase(M, G, MK_BC1, FBcond<T, 1>{0});
     grid.sync();
     if (G.tot[MK_BC2] > 0) {
-      group_phase(M, G, MK_BC2, FBcond<T, 2>{});
+      group_phase(M, G, MK_BC2, FBcond<T, 2>{0});
       grid.sync();
     }
   }
@@ -4167,7 +4295,7 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
 
 // explicit instantiations
 #define MGE_INST(T)                                                                                              \
-  template void launch_timestep<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t, bool);       \
+  template void launch_timestep<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t, bool, bool); \
   template void launch_solut<T>(const DevBlock<T>&, const PhysParams&, double, double, int, double*, cudaStream_t); \
   template void launch_stage<T>(const DevBlock<T>&, const PhysParams&, const StageArgs&, unsigned*, cudaStream_t,     \
                                 cudaStream_t, cudaEvent_t, cudaEvent_t);                                               \
@@ -4180,14 +4308,13 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   template void launch_irs<T>(const DevBlock<T>&, const PhysParams&, const IrsTables*, cudaStream_t, bool,       \
                               const int*, const StageArgs*);                                                    \
   template void launch_cutcell<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t);              \
-  template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t, bool);                     \
+  template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t, bool, unsigned*);          \
   template long long bc_items<T>(const DevBlock<T>&, int);                                                      \
   template long long split_items<T>(const DevBlock<T>&, int);                                                   \
   template void launch_rtrms<T>(const DevBlock<T>&, const PhysParams&, int, double*, int, double*, cudaStream_t, \
                                 unsigned*);                                                                    \
   template void launch_depvars_all<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                     \
   template void launch_copy_ws<T>(const DevBlock<T>&, cudaStream_t);                                            \
-  template void launch_save_wn<T>(const DevBlock<T>&, cudaStream_t);                                            \
   template void launch_copy_wn<T>(const DevBlock<T>&, cudaStream_t);                                            \
   template void launch_init_free<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                       \
   template void launch_forces<T>(const DevBlock<T>&, const double*, const double*, const double*, double, double*,  \

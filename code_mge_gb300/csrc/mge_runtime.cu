@@ -194,10 +194,10 @@ int check_err(mge_ctx* c) {
 }
 
 // ---------------------------------------------------------------- device ops
-void enqueue_timestep(mge_ctx* c, Block& b) {
+void enqueue_timestep(mge_ctx* c, Block& b, bool save = false) {
   with_dev(b, [&](auto& D) {
     using T = typename std::remove_reference_t<decltype(D)>::value_type;
-    launch_timestep<T>(D, c->P, c->d_err, c->stream, b.aux32);
+    launch_timestep<T>(D, c->P, c->d_err, c->stream, b.aux32, save);
   });
 }
 
@@ -267,29 +267,24 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
     if (rc == 0) return;
     cudaGetLastError();  // cooperative launch unavailable: fall through to per-phase launches
   }
-  // the time step (reads w, p; writes vdtim, lam, dtim) and the copies of w
-  // into ws and wn touch disjoint outputs: the copies run beside it
-  const bool copies_beside = with_timestep && c->side;
-  if (copies_beside) {
+  // the time step (reads w, p; writes vdtim, lam, dtim and wn = w) and the copy
+  // of w into ws touch disjoint outputs: the copy runs beside it
+  const bool copy_beside = with_timestep && lfir && c->side;
+  if (copy_beside) {
     cudaEventRecord(c->ev_fork, c->stream);
     cudaStreamWaitEvent(c->side, c->ev_fork, 0);
     with_dev(b, [&](auto& D) {
       using T = typename std::remove_reference_t<decltype(D)>::value_type;
-      if (lfir) launch_copy_ws<T>(D, c->side);
-      launch_save_wn<T>(D, c->side);
+      launch_copy_ws<T>(D, c->side);
     });
     cudaEventRecord(c->ev_join, c->side);
-    enqueue_timestep(c, b);
-    cudaStreamWaitEvent(c->stream, c->ev_join, 0);
-  } else if (with_timestep) {
-    enqueue_timestep(c, b);
   }
+  if (with_timestep) enqueue_timestep(c, b, true);
+  if (copy_beside) cudaStreamWaitEvent(c->stream, c->ev_join, 0);
   with_dev(b, [&](auto& D) {
     using T = typename std::remove_reference_t<decltype(D)>::value_type;
-    if (!copies_beside) {
-      if (lfir) launch_copy_ws<T>(D, c->stream);
-      launch_save_wn<T>(D, c->stream);
-    }
+    if (lfir && !copy_beside) launch_copy_ws<T>(D, c->stream);
+    if (!with_timestep) launch_copy_wn<T>(D, c->stream);
     for (int m = 1; m <= mstage; m++) {
       StageArgs A = stage_args(P, m, mgl, mlvl, lres, lfir, itime);
       A.fast = b.fast;
@@ -298,17 +293,8 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
       launch_stage<T>(D, c->P, A, c->d_err, c->stream, c->side, c->ev_fork, c->ev_join);
       if (lres) return;
       if (A.irs) launch_irs<T>(D, c->P, b.tabs, c->stream, b.aux32, b.irs_var, &A);
-      if (b.cut_beside_bcond && c->side) {  // disjoint data: the record pass beside the boundary passes
-        cudaEventRecord(c->ev_fork, c->stream);
-        cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-        launch_cutcell<T>(D, c->P, c->d_err, c->side);
-        cudaEventRecord(c->ev_join, c->side);
-        launch_bcond<T>(D, c->P, c->stream, faces_only);
-        cudaStreamWaitEvent(c->stream, c->ev_join, 0);
-      } else {
-        launch_cutcell<T>(D, c->P, c->d_err, c->stream);
-        launch_bcond<T>(D, c->P, c->stream, faces_only);
-      }
+      if (!b.cut_beside_bcond) launch_cutcell<T>(D, c->P, c->d_err, c->stream);
+      launch_bcond<T>(D, c->P, c->stream, faces_only, b.cut_beside_bcond ? c->d_err : nullptr);
     }
     if (want_rt) launch_rtrms<T>(D, c->P, P.vt, b.rt_partial, b.npart, b.rt_cur, c->stream, c->d_err);
   });
@@ -546,6 +532,7 @@ void fill_view(Block& b, DevBlock<T>& d, void* scratch) {
   d.rvolf = 1.0f / (float)b.vol;
   d.nmir = (int)b.recs.size();
   d.m0 = b.m0;
+  d.cut_beside = b.cut_beside_bcond;
   d.rec_i = b.rec_i; d.rec_cloud = b.rec_cloud; d.rec_coef = b.rec_coef; d.rec_nvec = b.rec_nvec;
   d.rec_qb = b.rec_qb; d.rec_area = b.rec_area; d.rec_wsol = (T*)b.rec_wsol; d.rec_psol = (T*)b.rec_psol;
   d.rec_wall = (T*)b.rec_wall; d.tgt_off = b.tgt_off; d.tgt_ops = b.tgt_ops;
@@ -579,12 +566,14 @@ int commit_block(mge_ctx* c, Block& b, double* scratch) {
   if ((rc = valloc(c, &b.w, 5 * N, es)) || (rc = valloc(c, &b.p, N, es)) || (rc = valloc(c, &b.wn, 5 * N, es)) ||
       (rc = valloc(c, &b.ws, 5 * N, es)) || (rc = valloc(c, &b.dw, 5 * N, es)) || (rc = valloc(c, &b.fw, 5 * N, es)) ||
       (rc = valloc(c, &b.wr, 5 * N, es)) || (rc = valloc(c, &b.qf, 5 * N, es)) || (rc = valloc(c, &b.vdtim, N, es)) ||
-      (rc = valloc(c, &b.lam, N, es)) || (rc = dalloc(c, &b.dtim, 1)) || (rc = dalloc(c, &b.blank, N)) ||
+      (rc = valloc(c, &b.lam, N, es)) || (rc = dalloc(c, &b.dtim, 3)) || (rc = dalloc(c, &b.blank, N)) ||
       (rc = dalloc(c, &b.marker, N)) || (rc = dalloc(c, &b.cutmap, N)))
     return rc;
   if (c->prm.irs_variant == 1 && (rc = valloc(c, &b.eps, 3 * N, es))) return rc;
   if (c->prm.execmode == 1 && ((rc = valloc(c, &b.w1, 5 * N, es)) || (rc = valloc(c, &b.w2, 5 * N, es)))) return rc;
   CK(cudaMemset(b.marker, 0, N));
+  const uint64_t dtim0[3] = {0, ~0ull, 0};  // no time step yet, the minimum of no blocks, no blocks
+  CK(cudaMemcpy(b.dtim, dtim0, sizeof(dtim0), cudaMemcpyHostToDevice));
   std::vector<uint8_t> bl(N);
   for (long long q = 0; q < N; q++) bl[q] = b.blank_h[q] != 0 ? 1 : 0;
   CK(cudaMemcpy(b.blank, bl.data(), N, cudaMemcpyHostToDevice));
@@ -1784,11 +1773,7 @@ int mge_kernel_times(mge_ctx* c, int level, int reps, double* ms_out, int nout) 
   };
   int rc = MGE_OK;
   for (int r = 0; r < reps && !rc; r++) {
-    rc = timed(0, [&] { enqueue_timestep(c, b); });
-    with_dev(b, [&](auto& D) {
-      using T = typename std::remove_reference_t<decltype(D)>::value_type;
-      launch_save_wn<T>(D, c->stream);
-    });
+    rc = timed(0, [&] { enqueue_timestep(c, b, true); });
     for (int m = 1; m <= P.mstage && !rc; m++) {
       StageArgs A;
       std::memset(&A, 0, sizeof(A));
@@ -1975,7 +1960,8 @@ void kind_counts(const Block& b, long long* n) {
   n[MK_FACE3] = b.f32 ? split_items(b.dev32, 1) : split_items(b.dev, 1);
   n[MK_N] = b.N;
   n[MK_N5] = 5 * b.N;
-  n[MK_REC] = (long long)b.recs.size();
+  n[MK_REC] = ((long long)b.recs.size() * 8 + 31) / 32 * 32;
+  n[MK_CUT] = b.cut_beside_bcond ? 0 : n[MK_REC];
   n[MK_IRS0] = 5 * ny * nz;
   n[MK_IRS1] = 5 * nx * nz;
   n[MK_IRS2] = 5 * nx * ny;

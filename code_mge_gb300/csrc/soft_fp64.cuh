@@ -216,5 +216,109 @@ MGE_SF_HD double div(double a, double b) {
   return from_bits(((A ^ B) & kSign) | (((uint64_t)(e - 1) << 52) + m));
 }
 
+// Several quotients by one divisor.  recip() keeps the divisor's significand and
+// the reciprocal of div()'s Newton steps; quot() and mulquot() then need one
+// 64-bit product for the estimate and one low product for the exact
+// remainder.
+struct Recip {
+  uint64_t x;     // 2^62 / D, D = m / 2^53 in [1/2, 1), to about 60 bits
+  uint64_t m;     // the divisor's significand, [2^52, 2^53)
+  uint32_t e;     // its biased exponent; 0 when it is not a normal number
+  uint32_t sign;  // its sign bit in place
+};
+
+MGE_SF_HD Recip recip(double b) {
+  const uint64_t B = bits(b);
+  Recip R;
+  R.m = (B & kFrac) | kOne;
+  R.e = (uint32_t)(B >> 52) & 0x7ffu;
+  if (R.e == 0x7ffu) R.e = 0;
+  R.sign = (uint32_t)(B >> 32) & 0x80000000u;
+  const uint64_t d = R.m << 11;
+#ifdef __CUDA_ARCH__
+  const float x0 = __frcp_rn((float)(uint32_t)(d >> 40) * 5.9604644775390625e-8f);  // 1 / (d_hi / 2^24)
+  const uint32_t xb = __float_as_uint(x0);
+#else
+  const float x0 = 1.0f / ((float)(uint32_t)(d >> 40) * 5.9604644775390625e-8f);
+  uint32_t xb;
+  memcpy(&xb, &x0, 4);
+#endif
+  uint64_t X = (uint64_t)((xb & 0x7fffffu) | 0x800000u) << (39 + ((xb >> 23) & 0xffu) - 127);
+  for (int it = 0; it < 2; it++) {
+    const uint64_t p = mulhi64(d, X);
+    if (p <= (1ull << 62)) {
+      X += mulhi64(X, ((1ull << 62) - p) << 2);
+    } else {
+      X -= mulhi64(X, (p - (1ull << 62)) << 2);
+    }
+  }
+  R.x = X;
+  return R;
+}
+
+// the high half of x*y to within three units, from three of its four partial products
+MGE_SF_HD uint64_t mulhi64_near(uint64_t x, uint64_t y) {
+  const uint32_t xl = (uint32_t)x, xh = (uint32_t)(x >> 32), yl = (uint32_t)y, yh = (uint32_t)(y >> 32);
+  return (uint64_t)xh * yh + (uint32_t)(((uint64_t)xh * yl) >> 32) + (uint32_t)(((uint64_t)xl * yh) >> 32);
+}
+
+// the rounded quotient's bits for a dividend of significand m in [2^52, 2^53)
+// and biased exponent ea, with the sign bit's word; false outside the normal range.
+// n estimates the 53-bit quotient to the nearest integer: R.x and the near product
+// are within a few units of 2^-62, far below half of n's unit, so n is at most one
+// off, and the exact remainder m 2^k - n R.m (below 2^54 in size) decides.  A
+// quotient of two 53-bit integers is never halfway between two 53-bit ones.
+MGE_SF_HD bool quot_bits(uint64_t m, int32_t ea, uint32_t sign, const Recip& R, uint64_t& out) {
+  const bool ge = m >= R.m;
+  const int32_t e = ea - (int32_t)R.e + (ge ? 1023 : 1022);
+  const uint64_t q = mulhi64_near(m << 11, R.x);
+  const uint32_t sh = ge ? 10u : 9u;
+  uint64_t n = (q + ((uint64_t)1 << (sh - 1))) >> sh;
+  const int64_t r2 = (int64_t)((m << (ge ? 53 : 54)) - ((n * R.m) << 1));  // twice the remainder
+  const int64_t half = (int64_t)R.m;
+  if (r2 > half) n += 1;
+  if (r2 < -half) n -= 1;
+  // packing: a quotient rounded up to 2^53 carries into the exponent
+  out = ((uint64_t)(sign ^ R.sign) << 32) | (((uint64_t)(uint32_t)(e - 1) << 52) + n);
+  return R.e != 0u && (uint32_t)(e - 1) < 2045u;
+}
+
+// a / b, R = recip(b)
+MGE_SF_HD double quot(double a, const Recip& R, double b) {
+  const uint64_t A = bits(a);
+  const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu;
+  uint64_t out;
+  if (!quot_bits((A & kFrac) | kOne, (int32_t)ea, (uint32_t)(A >> 32) & 0x80000000u, R, out) || ea - 1u >= 2046u)
+    return native_div(a, b);
+  return from_bits(out);
+}
+
+MGE_SF_NOINLINE double native_muldiv(double a, double b, double d) { return native_div(native_mul(a, b), d); }
+
+// (a * b) / d, each operation rounded, R = recip(d): mul() up to its packing,
+// then the quotient of the rounded significand
+MGE_SF_HD double mulquot(double a, double b, const Recip& R, double d) {
+  const uint64_t A = bits(a), B = bits(b);
+  const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu, eb = (uint32_t)(B >> 52) & 0x7ffu;
+  const int32_t e0 = (int32_t)(ea + eb) - 1023;
+  const uint64_t ma = (A & kFrac) | kOne, mb = (B & kFrac) | kOne;
+  const uint32_t al = (uint32_t)ma, ah = (uint32_t)(ma >> 32), bl = (uint32_t)mb, bh = (uint32_t)(mb >> 32);
+  const uint64_t t0 = (uint64_t)al * bl;
+  const uint64_t mid = (uint64_t)ah * bl + ((uint64_t)al * bh + (t0 >> 32));
+  const uint64_t hi = (uint64_t)ah * bh + (mid >> 32);
+  const uint64_t lo = (mid << 32) | (t0 & 0xffffffffull);
+  const uint32_t top = (uint32_t)(hi >> 41);
+  const uint32_t s = 12u - top;
+  uint64_t m = (hi << s) | (lo >> (64u - s));
+  const uint64_t rest = lo << s;
+  m += (rest >> 63) & ((uint64_t)((rest << 1) != 0) | (m & 1u));
+  const uint32_t carry = (uint32_t)(m >> 53);
+  m >>= carry;
+  uint64_t out;
+  const bool ok = quot_bits(m, e0 + (int32_t)(top + carry), (uint32_t)((A ^ B) >> 32) & 0x80000000u, R, out);
+  if (!ok || ea - 1u >= 2046u || eb - 1u >= 2046u || (uint32_t)(e0 - 1) >= 2044u) return native_muldiv(a, b, d);
+  return from_bits(out);
+}
+
 }  // namespace soft
 }  // namespace mge
