@@ -83,6 +83,22 @@ template <bool S, typename T> __device__ __forceinline__ T pdiv(T a, T b) {
 template <bool S, typename T> __device__ __forceinline__ T pmdiv(T a, T b, T y) {
   if constexpr (S) return smdiv(a, b, y); else return mdiv(a, b, y);
 }
+// Quotients by one divisor b: a/b and (a*w)/b, each operation rounded.  With the
+// integer pipes nothing is left on the FP64 pipe (soft::mulquot); without, one
+// reciprocal and Markstein's quotient.  The same bits as the divisions.
+template <bool S, typename T> struct SharedDiv {
+  T b, y;
+  __device__ __forceinline__ explicit SharedDiv(T d) : b(d), y(pdiv<S>(T(1), d)) {}
+  __device__ __forceinline__ T quot(T a) const { return pmdiv<S>(a, b, y); }
+  __device__ __forceinline__ T mulquot(T a, T w) const { return pmdiv<S>(pmul<S>(a, w), b, y); }
+};
+template <> struct SharedDiv<true, double> {
+  double b;
+  soft::Recip r;
+  __device__ __forceinline__ explicit SharedDiv(double d) : b(d), r(soft::recip(d)) {}
+  __device__ __forceinline__ double quot(double a) const { return soft::quot(a, r, b); }
+  __device__ __forceinline__ double mulquot(double a, double w) const { return soft::mulquot(a, w, r, b); }
+};
 // cell (or face) t of a box of nx by ny by any number of cells, counted from
 // (i0, i0, i0).  A block's scratch alone holds 64 fields, so its cells number
 // fewer than 2^31 on any device and 32-bit divisions suffice (a 64-bit one
@@ -158,14 +174,14 @@ __device__ __forceinline__ unsigned long long body_timestep(const DevBlock<T>& b
     for (int v = 0; v < 5; v++) b.wn[v * N + c] = b.w[v * N + c];
   }
   TC pc = (TC)b.p[c];
-  TC y = pdiv<S>(TC(1), w0);
-  TC cc = pmdiv<S>(pmul<S>(gamma, pc), w0, y);
+  const SharedDiv<S, TC> rho(w0);
+  TC cc = rho.mulquot(gamma, pc);
   if (cc < TC(0) || cc != cc) {  // timestep.f90:45-48
     atomicCAS(err, 0u, (unsigned)ERR_NEGPRESS);  // the first stop in launch order wins
     return mine;
   }
   cc = sqrt(fmaxT(cc, TC(0)));
-  TC uu = pmdiv<S>(w1, w0, y), uv = pmdiv<S>(w2, w0, y), uw = pmdiv<S>(w3, w0, y);
+  TC uu = rho.quot(w1), uv = rho.quot(w2), uw = rho.quot(w3);
   // face vectors are axis-aligned: |u.s| = |u_d s_d|, |s| precomputed
   TC ri = fabs(pmul<S>(uu, (TC)b.s[0])) + pmul<S>(cc, (TC)b.sqrt_ds[0]);
   TC rj = fabs(pmul<S>(uv, (TC)b.s[1])) + pmul<S>(cc, (TC)b.sqrt_ds[1]);
@@ -2747,15 +2763,20 @@ __device__ __forceinline__ bool fine_to_coarse(const Xfer& X, int ncp0, int ncp1
 }
 
 // the coarse correction w_c - ws_c of every coarse cell, formed once for the
-// 64 fine cells whose interpolation takes it (the same subtraction)
-template <typename TC>
-__device__ __forceinline__ void body_addw_diff(const DevBlock<TC>& c, double* dc, long long q) {
+// 64 fine cells whose interpolation takes it (the same subtraction).  TD: what
+// they take it as, FP32 for an FP64 level over an FP32 one: a conversion issues
+// at the FP64 rate, and 64 of them for each value took 1.8 of the mixed form's
+// 21 ms W-cycle at 192^3.
+template <typename TF, typename TC> struct Correction { typedef double type; };
+template <> struct Correction<double, float> { typedef float type; };
+template <typename TC, typename TD>
+__device__ __forceinline__ void body_addw_diff(const DevBlock<TC>& c, TD* dc, long long q) {
   if (q >= c.N) return;
 #pragma unroll
-  for (int v = 0; v < 5; v++) dc[v * c.N + q] = (double)c.w[v * c.N + q] - (double)c.ws[v * c.N + q];
+  for (int v = 0; v < 5; v++) dc[v * c.N + q] = (TD)((double)c.w[v * c.N + q] - (double)c.ws[v * c.N + q]);
 }
-template <typename TC>
-__global__ void k_addw_diff(DevBlock<TC> c, double* dc) {
+template <typename TC, typename TD>
+__global__ void k_addw_diff(DevBlock<TC> c, TD* dc) {
   body_addw_diff(c, dc, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -2763,10 +2784,7 @@ __global__ void k_addw_diff(DevBlock<TC> c, double* dc) {
 // dc holds w_c - ws_c (k_addw_diff) unless fmg
 template <typename TF, typename TC>
 __device__ __forceinline__ void body_addw(const DevBlock<TF>& f, const DevBlock<TC>& c, const Xfer& X, int fmg,
-                                          const double* dc, long long t) {
-  if (t >= (long long)f.nx * f.ny * f.nz) return;
-  int i, j, k;
-  cell_of(t, f.nx, f.ny, 2, i, j, k);
+                                          const typename Correction<TF, TC>::type* dc, int i, int j, int k) {
   if constexpr (std::is_same<TF, double>::value && std::is_same<TC, float>::value) {
     // the mixed form's finest level under an FP32 coarse level: the coarse
     // correction is FP32, so it is interpolated in FP32 (the same stencil
@@ -2794,7 +2812,7 @@ __device__ __forceinline__ void body_addw(const DevBlock<TF>& f, const DevBlock<
           for (int dj = 0; dj < 2; dj++)
             for (int di = 0; di < 2; di++) {
               const long long cq = cidx(c.Pi, c.Pj, sf[0] + di, sf[1] + dj, sf[2] + dk);
-              acc = fmaf((float)dc[v * c.N + cq], wx[di] * wy[dj] * wz[dk], acc);
+              acc = fmaf(dc[v * c.N + cq], wx[di] * wy[dj] * wz[dk], acc);
             }
         f.w[v * f.N + q] = f.w[v * f.N + q] + (double)acc;
       }
@@ -2825,8 +2843,91 @@ __device__ __forceinline__ void body_addw(const DevBlock<TF>& f, const DevBlock<
   }
 }
 template <typename TF, typename TC>
-__global__ void k_addw(DevBlock<TF> f, DevBlock<TC> c, Xfer X, int fmg, const double* dc) {
-  body_addw(f, c, X, fmg, dc, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void k_addw(DevBlock<TF> f, DevBlock<TC> c, Xfer X, int fmg, const typename Correction<TF, TC>::type* dc) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)f.nx * f.ny * f.nz) return;
+  int i, j, k;
+  cell_of(t, f.nx, f.ny, 2, i, j, k);
+  body_addw(f, c, X, fmg, dc, i, j, k);
+}
+
+// x / 64: the exponent less six where the result is normal (exact), else the product
+__device__ __forceinline__ double div64(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const unsigned e = (unsigned)hi & 0x7ff00000u;
+  if (e - 0x00700000u < 0x7f800000u) return __hiloint2double(hi - 0x00600000, lo);
+  return x * 0.015625;
+}
+// The 2:1 prolongation of FP64 arithmetic, eight fine cells a thread: the cells
+// 2m+1 and 2m+2 along each axis lie between the coarse centres s = o+m+1 and s+1,
+// so they share a stencil, and their weights 27, 9, 3 and 1 over 64 make four
+// products of each coarse value for all eight instead of one a cell each.  The
+// products round and add as a cell by itself forms them.  The fine cells along
+// the block's faces, whose stencil may be clamped, take k_addw_shell.  One cell
+// a thread spent about 100 FP64 operations on its weights, products and sums;
+// this spends 45 (1.0 ms less at 192^3).
+template <typename TF, typename TC>
+__global__ void __launch_bounds__(128) k_addw_octet(DevBlock<TF> f, DevBlock<TC> c, Xfer X, int fmg, const double* dc) {
+  const int n0 = f.nx / 2 - 1, n1 = f.ny / 2 - 1, n2 = f.nz / 2 - 1;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)n0 * n1 * n2) return;
+  int mi, mj, mk;
+  cell_of(t, n0, n1, 1, mi, mj, mk);
+  const long long q0 = cidx(c.Pi, c.Pj, X.o[0] + mi + 1, X.o[1] + mj + 1, X.o[2] + mk + 1);
+  const long long f0 = cidx(f.Pi, f.Pj, 2 * mi + 1, 2 * mj + 1, 2 * mk + 1);
+  const long long cj = c.Pi, ck = (long long)c.Pi * c.Pj, fj = f.Pi, fk = (long long)f.Pi * f.Pj;
+  bool fluid[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) fluid[e] = f.blank[f0 + (e & 1) + ((e >> 1) & 1) * fj + (e >> 2) * fk] != 0;
+#pragma unroll 1
+  for (int v = 0; v < 5; v++) {
+    double p[8][4];  // the coarse values times 27, 9, 3, 1 over 64
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      const long long q = q0 + (e & 1) + ((e >> 1) & 1) * cj + (e >> 2) * ck;
+      const double x = fmg ? (double)c.w[v * c.N + q] : dc[v * c.N + q];
+      p[e][0] = x * 0.421875;
+      p[e][1] = smul(x, 0.140625);
+      p[e][2] = smul(x, 0.046875);
+      p[e][3] = div64(x);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      // coarse value n is near fine cell e along the axes where their bits agree:
+      // weight 3/4 there, 1/4 where they differ
+      double acc = 0.0;
+#pragma unroll
+      for (int n = 0; n < 8; n++) {
+        const int far = ((n ^ e) & 1) + (((n ^ e) >> 1) & 1) + ((n ^ e) >> 2);
+        acc = n == 0 ? p[n][far] : acc + p[n][far];
+      }
+      const long long q = v * f.N + f0 + (e & 1) + ((e >> 1) & 1) * fj + (e >> 2) * fk;
+      if (fluid[e]) f.w[q] = fmg ? (TF)acc : (TF)((double)f.w[q] + acc);
+    }
+  }
+}
+// the fine cells on the block's six faces, one at a time
+template <typename TF>
+__host__ __device__ __forceinline__ long long shell_items(const DevBlock<TF>& f) {
+  return 2ll * f.nx * f.ny + 2ll * f.nx * (f.nz - 2) + 2ll * (f.ny - 2) * (f.nz - 2);
+}
+template <typename TF, typename TC>
+__global__ void k_addw_shell(DevBlock<TF> f, DevBlock<TC> c, Xfer X, int fmg, const double* dc) {
+  long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 >= shell_items(f)) return;
+  int t = (int)t0, i, j, k;
+  if (t < 2 * f.nx * f.ny) {
+    const int r = t % (f.nx * f.ny);
+    i = 2 + r % f.nx, j = 2 + r / f.nx, k = t < f.nx * f.ny ? 2 : f.kl;
+  } else if ((t -= 2 * f.nx * f.ny) < 2 * f.nx * (f.nz - 2)) {
+    const int n = f.nx * (f.nz - 2), r = t % n;
+    i = 2 + r % f.nx, k = 3 + r / f.nx, j = t < n ? 2 : f.jl;
+  } else {
+    t -= 2 * f.nx * (f.nz - 2);
+    const int n = (f.ny - 2) * (f.nz - 2), r = t % n;
+    j = 3 + r % (f.ny - 2), k = 3 + r / (f.ny - 2), i = t < n ? 2 : f.il;
+  }
+  body_addw(f, c, X, fmg, dc, i, j, k);
 }
 
 // bc_overlap.f90:32-90: ghost cell dst[t] of block g takes the trilinear
@@ -3283,136 +3384,157 @@ __device__ __forceinline__ int multi_case(const long long* off, int nc, long lon
   return sq;
 }
 
+// Blocks of 256 threads an SM is asked to hold for a phase (registers are cut to
+// fit), as the phase's own kernel has it
+template <typename F> struct MinBlocks { static constexpr int v = 4; };
+// A thread block's case is copied to shared memory first: read from the group's
+// array in global memory, every field would be loaded again after each store
+// that might have changed it.
 template <typename T, typename F>
-__global__ void __launch_bounds__(256) k_multi(MultiArgs<T> M, F f) {
+__global__ void __launch_bounds__(256, MinBlocks<F>::v) k_multi(MultiArgs<T> M, F f) {
+  __shared__ DevBlock<T> sb;
+  __shared__ PhysParams sp;
+  static_assert(sizeof(DevBlock<T>) % 4 == 0 && sizeof(PhysParams) % 4 == 0, "copied by words");
   const long long base = (long long)blockIdx.x * 256;
   const int q = multi_case(M.off, M.nc, base);
-  f(M, q, base - M.off[q] + threadIdx.x);
+  for (int w = threadIdx.x; w < (int)(sizeof(DevBlock<T>) / 4); w += 256) ((int*)&sb)[w] = ((const int*)(M.B + q))[w];
+  for (int w = threadIdx.x; w < (int)(sizeof(PhysParams) / 4); w += 256) ((int*)&sp)[w] = ((const int*)(M.P + q))[w];
+  __syncthreads();
+  f(M, q, base - M.off[q] + threadIdx.x, sb, sp);
 }
 
 template <typename T, typename TC, bool S> struct FTimestep {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     unsigned long long mine = ~0ull;
     const long long n = (long long)b.nx * b.ny * b.nz;
-    if (t < n) mine = body_timestep<T, TC, S, true>(b, M.P[q], M.err[q], t);
+    if (t < n) mine = body_timestep<T, TC, S, true>(b, P, M.err[q], t);
     block_min_dtim(mine, b.dtim, (int)((n + 255) / 256));  // a call per 256 cells, whichever block makes it
   }
 };
 template <typename T> struct FCopyWs {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     if (t < 5 * b.N) b.ws[t] = b.w[t];
   }
 };
 template <typename T, bool FAST, bool S> struct FPrep {
   int dissip_on;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, FAST, S>(b, M.P[q], dissip_on, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    if (t < (long long)b.ie * b.je * b.ke) body_prep<T, FAST, S>(b, P, dissip_on, t);
   }
 };
 template <typename T, bool S> struct FFace {
   int dissip_on;
   T cd;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
-    if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL, S>(b, M.P[q], dissip_on, cd, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    if (t < (long long)(b.ie - 1) * (b.je - 1) * (b.ke - 1)) body_face<T, FACE_CENTRAL, S>(b, P, dissip_on, cd, t);
   }
 };
 template <typename T> struct FFaceConv {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const { body_face_conv(M.B[q], t); }
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const { body_face_conv(b, t); }
 };
 template <typename T, bool FAST, bool S> struct FPrepRows {
   int dissip_on;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    body_prep_rows<T, FAST, S>(M.B[q], M.P[q], dissip_on, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    body_prep_rows<T, FAST, S>(b, P, dissip_on, t);
   }
 };
 template <typename T, bool FAST, bool S> struct FFaceRows {
   int dissip_on;
   T cd;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    body_face_rows<T, FAST, S>(M.B[q], M.P[q], dissip_on, cd, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    body_face_rows<T, FAST, S>(b, P, dissip_on, cd, t);
   }
 };
 template <typename T> struct FRec {
   int dissip_on;
   T cd;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    if (split_scheme(M.P[q])) {
-      if (t < rec_lane_items(M.B[q])) rec_wall_lanes(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
-    } else if (t < M.B[q].nmir) {
-      rec_wall_terms(M.B[q], M.P[q], dissip_on, cd, M.err[q], (int)t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    if (split_scheme(P)) {
+      if (t < rec_lane_items(b)) rec_wall_lanes(b, P, dissip_on, cd, M.err[q], (int)t);
+    } else if (t < b.nmir) {
+      rec_wall_terms(b, P, dissip_on, cd, M.err[q], (int)t);
     }
   }
 };
 template <typename T, bool FAST, bool S> struct FCombine {
   StageArgs A;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST, S>(b, M.P[q], A, M.err[q], t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    if (t < (long long)b.nx * b.ny * b.nz) body_combine<T, FAST, S>(b, P, A, M.err[q], t);
   }
 };
 template <typename T, typename TC, int D> struct FIrs {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     if (t >= 5 * irs_lines<T, D>(b)) return;
     if constexpr (std::is_same<TC, double>::value) {
       if (M.tab[3 * q + D].quick) {
-        body_irs<T, TC, D, false, true>(b, M.tab[3 * q + D], (TC)(-M.P[q].smoo), t);
+        body_irs<T, TC, D, false, true>(b, M.tab[3 * q + D], (TC)(-P.smoo), t);
         return;
       }
     }
-    body_irs<T, TC, D>(b, M.tab[3 * q + D], (TC)(-M.P[q].smoo), t);
+    body_irs<T, TC, D>(b, M.tab[3 * q + D], (TC)(-P.smoo), t);
   }
 };
 // the mixed form's finest level: FP32 sweeps on one FP32 copy of dw (in F)
 template <typename TS, typename TO, int D> struct FIrsMixed {
-  __device__ void operator()(const MultiArgs<double>& M, int q, long long t) const {
-    const DevBlock<double>& b = M.B[q];
+  __device__ void operator()(const MultiArgs<double>& M, int q, long long t, const DevBlock<double>& b,
+                             const PhysParams& P) const {
     if (t >= 5 * irs_lines<double, D>(b)) return;
     float* cp = (float*)b.F;
     const TS* src = D == 0 ? (const TS*)b.dw : (const TS*)cp;
     TO* out = D == 2 ? (TO*)b.dw : (TO*)cp;
-    body_irs_mixed<TS, TO, D>(b, M.tab[3 * q + D], (float)(-M.P[q].smoo), src, cp, out, t);
+    body_irs_mixed<TS, TO, D>(b, M.tab[3 * q + D], (float)(-P.smoo), src, cp, out, t);
   }
 };
 template <typename T, bool S> struct FUpdate {
   StageArgs A;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
-    if (t < (long long)b.nx * b.ny * b.nz) body_update<T, S>(b, M.P[q], A, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    if (t < (long long)b.nx * b.ny * b.nz) body_update<T, S>(b, P, A, t);
   }
 };
 template <typename T> struct FCutcell {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     // the blocks whose records do not share the boundary launch
-    if (!M.B[q].cut_beside && t < rec_lane_items(M.B[q])) cutcell_lanes(M.B[q], M.P[q], M.err[q], (int)t);
+    if (!b.cut_beside && t < rec_lane_items(b)) cutcell_lanes(b, P, M.err[q], (int)t);
   }
 };
 template <typename T, int PART> struct FBcond {
   int cut;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    body_bcond<T, PART>(M.B[q], M.P[q], M.err[q], cut, t);
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    body_bcond<T, PART>(b, P, M.err[q], cut, t);
   }
 };
 template <typename T> struct FDepvars {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const { body_depvars(M.B[q], M.P[q].gamma, t); }
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const { body_depvars(b, P.gamma, t); }
 };
 template <typename T> struct FCopyWn {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const { body_copy_wn(M.B[q], t); }
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const { body_copy_wn(b, t); }
 };
 // residual partial sums: thread block (case, part), 256 threads each
 template <typename T> struct FRtrmsPartial {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     const int part = (int)(t / 256);
-    if (part < M.npart[q]) body_rtrms_partial(M.B[q], M.P[q].cfl, M.P[q].vt, M.rt_partial[q], M.npart[q], part);
+    if (part < M.npart[q]) body_rtrms_partial(b, P.cfl, P.vt, M.rt_partial[q], M.npart[q], part);
   }
 };
 template <typename T> struct FRtrmsFinal {
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
-    const DevBlock<T>& b = M.B[q];
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
     if (t < 32) body_rtrms_final(M.rt_partial[q], M.npart[q], (double)b.nx * b.ny * b.nz, M.rt_out[q], M.err[q]);
   }
 };
@@ -3447,13 +3569,17 @@ template <typename TC, typename TF> struct FCollc {
 };
 template <typename TC, typename TF> struct FAddwDiff {
   __device__ void operator()(const MultiPairArgs<TC, TF>& M, int q, long long t) const {
-    body_addw_diff(M.C[q], M.dc[q], t);
+    body_addw_diff(M.C[q], (typename Correction<TF, TC>::type*)M.dc[q], t);
   }
 };
 template <typename TC, typename TF> struct FAddw {
   int fmg;
   __device__ void operator()(const MultiPairArgs<TC, TF>& M, int q, long long t) const {
-    body_addw(M.F[q], M.C[q], M.X[q], fmg, M.dc[q], t);
+    const DevBlock<TF>& f = M.F[q];
+    if (t >= (long long)f.nx * f.ny * f.nz) return;
+    int i, j, k;
+    cell_of(t, f.nx, f.ny, 2, i, j, k);
+    body_addw(f, M.C[q], M.X[q], fmg, (const typename Correction<TF, TC>::type*)M.dc[q], i, j, k);
   }
 };
 template <typename TC, typename TF> struct FEmbed {
@@ -3461,6 +3587,19 @@ template <typename TC, typename TF> struct FEmbed {
     body_embed(M.F[q], M.C[q], M.X[q], M.P[q].gamma, t);
   }
 };
+
+// measured on eight mixed cases of 32^3 to 96^3: the contracted combine 345 us at 4,
+// 336 at 5; the prep 270, 257; the dissipation faces 373 at 1 to 5, 337 at 6; the FP32
+// faces 60, 44; the i sweep 223, 207 at 1
+template <bool S> struct MinBlocks<FCombine<double, true, S>> { static constexpr int v = 5; };
+template <bool S> struct MinBlocks<FPrep<double, true, S>> { static constexpr int v = 5; };
+template <bool S> struct MinBlocks<FFaceRows<double, true, S>> { static constexpr int v = 6; };
+template <bool S> struct MinBlocks<FFace<float, S>> { static constexpr int v = 5; };
+template <> struct MinBlocks<FIrsMixed<double, float, 0>> { static constexpr int v = 1; };
+template <typename T, typename TC, bool S> struct MinBlocks<FTimestep<T, TC, S>> { static constexpr int v = 6; };
+// the plain forms as in their own kernels
+template <> struct MinBlocks<FPrep<double, false, true>> { static constexpr int v = 6; };
+template <typename T, int D> struct MinBlocks<FIrs<T, T, D>> { static constexpr int v = 3; };
 
 // =============================================================== launchers
 constexpr int TPB = 256;
@@ -3919,8 +4058,27 @@ void launch_addw(const DevBlock<TF>& f, const DevBlock<TC>& c, const int ratio[3
   long long n = (long long)f.nx * f.ny * f.nz;
   // the coarse corrections go to the stage scratch (at least 64 fields of
   // the largest block), free between euler calls
-  if (!fmg) k_addw_diff<TC><<<LAUNCH_N(c.N), 0, s>>>(c, scratch);
-  k_addw<TF, TC><<<LAUNCH_N(n), 0, s>>>(f, c, X, fmg, scratch);
+  typedef typename Correction<TF, TC>::type TD;
+  TD* dc = (TD*)scratch;
+  if (!fmg) k_addw_diff<TC, TD><<<LAUNCH_N(c.N), 0, s>>>(c, dc);
+  if constexpr (std::is_same<TD, double>::value) {
+    // whole 2:1 coarsening, the fine block inside its parent: eight cells a
+    // thread, from the size on at which the saved products outweigh the second
+    // launch (a W-cycle with 192^3 finest 37.1 against 38.1 ms, 64^3 3.29 against 3.31; the
+    // 48^3 level of a mixed hierarchy 0.46 against 0.45)
+    bool octets = n > 200000;
+    const int nf[3] = {f.nx, f.ny, f.nz}, nc[3] = {c.nx, c.ny, c.nz};
+    for (int d = 0; d < 3; d++)
+      octets = octets && X.r[d] == 2 && X.o[d] >= 0 && nf[d] >= 4 && nf[d] % 2 == 0 && X.o[d] + nf[d] / 2 <= nc[d];
+    if (octets) {
+      const long long no = (long long)(f.nx / 2 - 1) * (f.ny / 2 - 1) * (f.nz / 2 - 1);
+      const int to = std::min(tpb_for(no), 128);
+      k_addw_octet<TF, TC><<<nblk(no, to), to, 0, s>>>(f, c, X, fmg, dc);
+      k_addw_shell<TF, TC><<<LAUNCH_N(shell_items(f)), 0, s>>>(f, c, X, fmg, dc);
+      return;
+    }
+  }
+  k_addw<TF, TC><<<LAUNCH_N(n), 0, s>>>(f, c, X, fmg, dc);
 }
 
 template <typename TF, typename TC>
@@ -4040,7 +4198,7 @@ static void multi_euler_t(const MultiLevel& L, const StageArgs* A, int mstage, b
 template <typename T> struct FGather {
   double* res;
   unsigned* errs;
-  __device__ void operator()(const MultiArgs<T>& M, int q, long long t) const {
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>&, const PhysParams&) const {
     if (t == 0) {
       res[q] = *M.rt_out[q];
       errs[q] = *M.err[q];
@@ -4085,7 +4243,7 @@ __device__ __forceinline__ void group_phase(const MultiArgs<T>& M, const GroupEu
   const long long tot = G.tot[kind];
   for (long long base = (long long)blockIdx.x * 256; base < tot; base += (long long)gridDim.x * 256) {
     const int q = case_of(G.off[kind], M.nc, base);
-    f(M, q, base - G.off[kind][q] + threadIdx.x);
+    f(M, q, base - G.off[kind][q] + threadIdx.x, M.B[q], M.P[q]);
   }
 }
 

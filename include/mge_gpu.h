@@ -221,7 +221,7 @@ int mge_prolong_async(mge_ctx* ctx, int mlvl);
  * record, combine passes, the line sweeps, the boundary passes, the
  * transfers) is one launch over the block of that level of every case; on a
  * level whose blocks hold at most MGE_GROUP_COOP_MAX_CELLS cells in all
- * (environment, 300,000 by default) the whole update of every case is one
+ * (environment, 0 by default: none) the whole update of every case is one
  * persistent cooperative launch instead.  The whole cycle is one captured
  * CUDA graph, so the launches of a cycle do not grow with the number of
  * cases.  The reference's solver loops the
