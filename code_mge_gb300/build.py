@@ -15,7 +15,14 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libmge_gpu.so")
 ROOT = os.path.dirname(HERE)
-SOURCES = ["mge_kernels.cu", "mge_runtime.cu", "mge_noalloc.cu", "mge_restart.cpp"]
+# (source, object, its own flags); the kernels in three parts (MGE_PART), so
+# that they compile side by side
+SOURCES = [("mge_kernels.cu", "mge_kernels_f64.o", ["-DMGE_PART=0"]),
+           ("mge_kernels.cu", "mge_kernels_f32.o", ["-DMGE_PART=1"]),
+           ("mge_kernels.cu", "mge_kernels_group.o", ["-DMGE_PART=2"]),
+           ("mge_runtime.cu", "mge_runtime.o", []),
+           ("mge_noalloc.cu", "mge_noalloc.o", []),
+           ("mge_restart.cpp", "mge_restart.o", [])]
 HEADERS = ["mge_internal.h", "exact_ops.cuh", "fast_pow.cuh", "soft_fp64.cuh", "quick_quotient.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "--fmad=false", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
@@ -37,12 +44,11 @@ def build(force=False, verbose=False):
     os.makedirs(OUT_DIR, exist_ok=True)
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "mge_gpu.h")]
     objs, jobs = [], []
-    for s in SOURCES:
-        src = os.path.join(CSRC, s)
-        obj = os.path.join(OUT_DIR, os.path.splitext(s)[0] + ".o")
+    for s, o, flags in SOURCES:
+        src, obj = os.path.join(CSRC, s), os.path.join(OUT_DIR, o)
         objs.append(obj)
         if force or _stale(obj, [src] + hdrs):
-            jobs.append([_nvcc()] + ARCH + NVCC_FLAGS + ["-c", src, "-o", obj])
+            jobs.append([_nvcc()] + ARCH + NVCC_FLAGS + flags + ["-c", src, "-o", obj])
 
     def run(cmd):
         if verbose:

@@ -39,6 +39,13 @@
 
 namespace cg = cooperative_groups;
 
+// The file is compiled once per part, in parallel: 0 the launchers on FP64
+// blocks (and what belongs to no precision), 1 those on FP32 blocks, 2 the
+// launches over several cases.
+#ifndef MGE_PART
+#error "compile with -DMGE_PART=0, 1 and 2"
+#endif
+
 namespace mge {
 
 // --------------------------------------------------------------- helpers
@@ -2527,11 +2534,13 @@ __global__ void k_bcond(DevBlock<T> b, PhysParams P, unsigned* err, int cut) {
 // --------------------------------------------------------------- residual norm (euler.f90:431-447)
 // Deterministic: fixed partial ranges, fixed-order tree per block, one final block.
 constexpr int RT_THREADS = 256;
+#if MGE_PART == 0
 int rtrms_partials(long long ncells) {
   long long per = (long long)RT_THREADS * 8;
   long long n = (ncells + per - 1) / per;
   return (int)(n < 1 ? 1 : (n > 4096 ? 4096 : n));
 }
+#endif
 
 template <typename T>
 __device__ void body_rtrms_partial(const DevBlock<T>& b, double cfl, int vt, double* partial, int npart, int part) {
@@ -2583,7 +2592,7 @@ __device__ __forceinline__ void body_rtrms_final(const double* partial, int npar
   }
 }
 
-__global__ void k_rtrms_final(const double* partial, int npart, double ncell, double* out, unsigned* err) {
+static __global__ void k_rtrms_final(const double* partial, int npart, double ncell, double* out, unsigned* err) {
   if (blockIdx.x == 0 && threadIdx.x < 32) body_rtrms_final(partial, npart, ncell, out, err);
 }
 
@@ -3910,10 +3919,12 @@ template <typename T>
 long long split_items(const DevBlock<T>& b, int e) {
   return split_items_t(b, e);
 }
+#if MGE_PART == 0
 void split_passes(const PhysParams& P, bool fast, long long cells, bool* prep, bool* face) {
   *prep = split_scheme(P) && split_prep(fast, cells);
   *face = split_scheme(P) && split_face(fast, cells);
 }
+#endif
 
 template <typename T>
 void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* partial, int npartial, double* out,
@@ -3922,6 +3933,7 @@ void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* par
   k_rtrms_final<<<1, 32, 0, s>>>(partial, npartial, (double)b.nx * b.ny * b.nz, out, err);
 }
 
+#if MGE_PART == 0
 template <typename TS, typename TD>
 __global__ void k_convert(const TS* __restrict__ a, TD* __restrict__ b, long long n) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -3949,19 +3961,25 @@ void launch_movsurf(long long nmir, const double* psurf, double* pnew, double* q
   if (nmir <= 0) return;
   k_movsurf<<<nblk(3 * nmir, TPB), TPB, 0, s>>>(3 * nmir, psurf, pnew, qb, vel_fs);
 }
+#endif
 
 // opt-in shared memory of the tiled line sweeps; called once per device at set-up
-void init_kernel_attributes() {
+void init_kernel_attributes_f32();
 #define MGE_SMEM_ATTR(T, TC)                                                                                     \
   cudaFuncSetAttribute(k_irs_smem<T, TC, 0, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);     \
   cudaFuncSetAttribute(k_irs_smem<T, TC, 1, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);     \
   cudaFuncSetAttribute(k_irs_smem<T, TC, 2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+#if MGE_PART == 0
+void init_kernel_attributes() {
   MGE_SMEM_ATTR(double, double)
   MGE_SMEM_ATTR(double, float)
-  MGE_SMEM_ATTR(float, float)
-#undef MGE_SMEM_ATTR
   cudaFuncSetAttribute(k_irs_smem_fill<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  init_kernel_attributes_f32();
 }
+#elif MGE_PART == 1
+void init_kernel_attributes_f32() { MGE_SMEM_ATTR(float, float) }
+#endif
+#undef MGE_SMEM_ATTR
 
 // grid of the cooperative kernel: every block resident at once
 template <typename T, typename TA>
@@ -4101,6 +4119,7 @@ void launch_forces(const DevBlock<T>& b, const double* origin, const double* h, 
                                 mu, out7);
 }
 
+#if MGE_PART == 2
 // --------------------------------------------------------------- a group's lockstep steps
 size_t xfer_size() { return sizeof(Xfer); }
 void make_xfer_host(const int ratio[3], const int offset[3], void* out) {
@@ -4451,6 +4470,8 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   });
 }
 
+#else
+
 // explicit instantiations
 #define MGE_INST(T)                                                                                              \
   template void launch_timestep<T>(const DevBlock<T>&, const PhysParams&, unsigned*, cudaStream_t, bool, bool); \
@@ -4479,8 +4500,11 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
                                  cudaStream_t);                                                                  \
   template void launch_overlap<T>(const DevBlock<T>&, const DevBlock<T>&, const long long*, const long long*,        \
                                   const double*, long long, const PhysParams&, cudaStream_t);
+#if MGE_PART == 0
 MGE_INST(double)
+#else
 MGE_INST(float)
+#endif
 #undef MGE_INST
 #define MGE_XFER(TC, TF)                                                                                         \
   template void launch_collc<TC, TF>(const DevBlock<TC>&, const DevBlock<TF>&, const int*, const int*, uint8_t*,   \
@@ -4489,10 +4513,14 @@ MGE_INST(float)
                                     double*, cudaStream_t);                                                     \
   template void launch_embed<TF, TC>(const DevBlock<TF>&, const DevBlock<TC>&, const int*, const int*,              \
                                      const PhysParams&, cudaStream_t);
+#if MGE_PART == 0
 MGE_XFER(double, double)
 MGE_XFER(float, double)
+#else
 MGE_XFER(float, float)
+#endif
 #undef MGE_XFER
+#endif  // MGE_PART == 2
 
 
 }  // namespace mge

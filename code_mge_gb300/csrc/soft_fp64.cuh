@@ -26,7 +26,7 @@
 
 #ifdef __CUDACC__
 #define MGE_SF_HD __host__ __device__ __forceinline__
-#define MGE_SF_NOINLINE __host__ __device__ __noinline__
+#define MGE_SF_NOINLINE __host__ __device__ __noinline__ inline
 #else
 #define MGE_SF_HD inline
 #define MGE_SF_NOINLINE inline
