@@ -199,6 +199,7 @@ struct MultiLevel {
 enum MultiPairKind { MP_COLLC = 0, MP_CN, MP_FPHYS, MP_FN, MP_COUNT };
 struct MultiPair {
   int nc = 0;
+  bool embed = true;             // some case has ghost cells inside its parent (bc_embed)
   bool c32 = false, f32 = false;
   void* C = nullptr;             // DevBlock<TC>[nc]
   void* F = nullptr;             // DevBlock<TF>[nc]
@@ -253,6 +254,8 @@ template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& 
 template <typename T> void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename T> void launch_copy_ws(const DevBlock<T>& b, cudaStream_t s);
 template <typename T> void launch_copy_wn(const DevBlock<T>& b, cudaStream_t s);
+// depvars on every cell, and wn = w on the physical ones (movco.f90:27-35)
+template <typename T> void launch_depvars_wn(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename T> void launch_init_free(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename TC, typename TF>
 void launch_collc(const DevBlock<TC>& c, const DevBlock<TF>& f, const int ratio[3], const int offset[3],

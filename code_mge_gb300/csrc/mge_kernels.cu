@@ -9,9 +9,9 @@
 //   k_prep     per cell: 1/rho, rho*E+p, the cell flux F(w).s for i/j/k
 //              (ceflux, eflux.f90:133-155) and the pressure sensors
 //              (dflux.f90:71-76,131-136,188-193)
-//   k_face     per face: averaged convective flux (eflux.f90:42-98) and the
+//   k_face_*   per face: averaged convective flux (eflux.f90:42-98) and the
 //              blended 2nd/4th-difference dissipation (dflux.f90:82-112)
-//   k_rec      per cut-cell record: the efluxb/dfluxb face replacements
+//   k_rec_*    per cut-cell record: the efluxb/dfluxb face replacements
 //   k_combine  per cell: dw, fw, forcing, blanking, time-step scaling and,
 //              without smoothing, the update + depvars (euler.f90:127-399)
 //   k_irs_*    implicit residual smoothing lines (psmoo.f90:171-237), the
@@ -2627,6 +2627,25 @@ __device__ __forceinline__ void body_copy_wn(const DevBlock<T>& b, long long c) 
   if (!(i >= 2 && i <= b.il && j >= 2 && j <= b.jl && k >= 2 && k <= b.kl)) return;
   for (int v = 0; v < 5; v++) b.wn[v * b.N + c] = b.w[v * b.N + c];
 }
+// depvars on every cell and wn = w on the physical ones, from one read of w
+template <typename T>
+__device__ __forceinline__ void body_depvars_wn(const DevBlock<T>& b, double gamma, long long c) {
+  if (c >= b.N) return;
+  int i, j, k;
+  cell_of(c, b.Pi, b.Pj, 0, i, j, k);
+  const bool phys = i >= 2 && i <= b.il && j >= 2 && j <= b.jl && k >= 2 && k <= b.kl;
+  T wv[5];
+#pragma unroll
+  for (int v = 0; v < 5; v++) {
+    wv[v] = b.w[v * b.N + c];
+    if (phys) b.wn[v * b.N + c] = wv[v];
+  }
+  b.p[c] = depvars((T)gamma, wv);
+}
+template <typename T>
+__global__ void k_depvars_wn(DevBlock<T> b, double gamma) {
+  body_depvars_wn(b, gamma, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
 template <typename T>
 __global__ void k_copy_wn(DevBlock<T> b) {
   body_copy_wn(b, (long long)blockIdx.x * blockDim.x + threadIdx.x);
@@ -3529,6 +3548,12 @@ template <typename T> struct FDepvars {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
                              const PhysParams& P) const { body_depvars(b, P.gamma, t); }
 };
+template <typename T> struct FDepvarsWn {
+  __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
+                             const PhysParams& P) const {
+    body_depvars_wn(b, P.gamma, t);
+  }
+};
 template <typename T> struct FCopyWn {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
                              const PhysParams& P) const { body_copy_wn(b, t); }
@@ -3566,11 +3591,6 @@ __global__ void __launch_bounds__(256) k_multi2(MultiPairArgs<TC, TF> M, Fn f) {
   const int q = multi_case(M.off, M.nc, base);
   f(M, q, base - M.off[q] + threadIdx.x);
 }
-template <typename TC, typename TF> struct FMarkerClear {
-  __device__ void operator()(const MultiPairArgs<TC, TF>& M, int q, long long t) const {
-    if (t < M.C[q].N) M.marker[q][t] = 0;
-  }
-};
 template <typename TC, typename TF> struct FCollc {
   __device__ void operator()(const MultiPairArgs<TC, TF>& M, int q, long long t) const {
     body_collc(M.C[q], M.F[q], M.X[q], M.marker[q], t);
@@ -4032,12 +4052,17 @@ int launch_euler_coop(const DevBlock<T>& b, const PhysParams& P, const EulerLaun
 
 template <typename T>
 void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s) {
-  k_depvars_all<T><<<nblk(b.N, TPB), TPB, 0, s>>>(b, P.gamma);
+  k_depvars_all<T><<<LAUNCH_N(b.N), 0, s>>>(b, P.gamma);
 }
 
 template <typename T>
 void launch_copy_ws(const DevBlock<T>& b, cudaStream_t s) {
   k_copy5<T><<<nblk(5 * b.N, TPB), TPB, 0, s>>>(b.w, b.ws, 5 * b.N);
+}
+
+template <typename T>
+void launch_depvars_wn(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s) {
+  k_depvars_wn<T><<<LAUNCH_N(b.N), 0, s>>>(b, P.gamma);
 }
 
 template <typename T>
@@ -4438,14 +4463,12 @@ void multi_movco_level(const MultiLevel& L, const MultiPair* pair, cudaStream_t 
       using TC = std::remove_pointer_t<decltype(tc)>;
       using TF = std::remove_pointer_t<decltype(tf)>;
       MultiPairArgs<TC, TF> M = pair_args<TC, TF>(*pair);
-      go_pair(*pair, M, MP_CN, FMarkerClear<TC, TF>{}, s);
       go_pair(*pair, M, MP_COLLC, FCollc<TC, TF>{}, s);
     });
   auto rest = [&](auto* tp) {
     using T = std::remove_pointer_t<decltype(tp)>;
     MultiArgs<T> M = multi_args<T>(L);
-    go_multi(L, M, MK_N, FDepvars<T>{}, s);
-    go_multi(L, M, MK_N, FCopyWn<T>{}, s);
+    go_multi(L, M, MK_N, FDepvarsWn<T>{}, s);
     multi_bcond(L, M, s);
   };
   if (L.f32)
@@ -4465,7 +4488,7 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
     go_pair(pair, M, MP_FPHYS, FAddw<TC, TF>{fmg ? 1 : 0}, s);
     MultiArgs<TF> F = multi_args<TF>(L);
     go_multi(L, F, MK_N, FDepvars<TF>{}, s);
-    go_pair(pair, M, MP_FN, FEmbed<TC, TF>{}, s);
+    if (pair.embed) go_pair(pair, M, MP_FN, FEmbed<TC, TF>{}, s);
     multi_bcond(L, F, s);
   });
 }
@@ -4495,6 +4518,7 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   template void launch_depvars_all<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                     \
   template void launch_copy_ws<T>(const DevBlock<T>&, cudaStream_t);                                            \
   template void launch_copy_wn<T>(const DevBlock<T>&, cudaStream_t);                                            \
+  template void launch_depvars_wn<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                      \
   template void launch_init_free<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                       \
   template void launch_forces<T>(const DevBlock<T>&, const double*, const double*, const double*, double, double*,  \
                                  cudaStream_t);                                                                  \
