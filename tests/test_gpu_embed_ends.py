@@ -12,7 +12,7 @@ from code_mge_gb300 import cases as K
 from code_mge_gb300.runtime import Cycle
 from oracle.oracle import OracleCycle
 from tests.parity import RTOL, rel_err
-from tests.test_gpu_group import _fmg_group, _fmg_single, _open
+from tests.test_gpu_group import _fmg_group, _fmg_single
 
 pytestmark = pytest.mark.gpu
 
@@ -66,7 +66,9 @@ def test_embed_ends(ends):
 
 def test_group_asks_all_its_cases(gpulib, monkeypatch):
     cases = [_case("all_on"), _case("inside")]
-    single, group = _open(cases, monkeypatch), _open(cases, monkeypatch)
+    monkeypatch.setenv("MGE_TUNE_PLAN", "1:0000,2:0000")
+    monkeypatch.setenv("MGE_COOP_MAX_CELLS", "0")
+    single, group = [Cycle(c) for c in cases], [Cycle(c) for c in cases]
     hs = [_fmg_single(gpulib, c, k) for c, k in zip(single, cases)]
     hg = _fmg_group(gpulib, group, cases)
     for q in range(len(cases)):
