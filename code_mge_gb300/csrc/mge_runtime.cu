@@ -362,7 +362,7 @@ void enqueue_overlap(mge_ctx* c, int mgl) {
 // parent.  Along an axis the ghosts below lie in it when the child starts
 // inside (offset > 0), those above when it ends inside; with both its ends on
 // the parent's in every axis there is none, and the launch over the block's cells
-// is left out (it and the two launches fewer of movco: 48^3 W-cycle 2.66 -> 2.61 ms).
+// is left out (it and the two launches fewer of movco: 48^3 W-cycle 2.66 -> 2.64 ms).
 bool embed_has_cells(const Block& f, const Block& pb) {
   const int n[3] = {f.nx, f.ny, f.nz}, np[3] = {pb.nx, pb.ny, pb.nz};
   for (int d = 0; d < 3; d++)
