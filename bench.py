@@ -45,11 +45,11 @@ UNIT = "cell-updates/s"
 # 5-variable fields of 40 B): smoothing stages 11 fields, non-smoothing
 # stages 4 fields, 17 B of scalars per stage, 56 B for the time step.
 BYTES_PER_CELL_UPDATE_IRS = (11 + 4 + 11 + 4 + 11) * 40 + 5 * 17 + 56   # 1,781
-# The roofline kernel is k_face on a stage with dissipation (stage 1), one
-# thread per cell of [2..ie]^3.  Compulsory bytes per cell: it reads the
-# per-cell fluxes F (15), sensors (3), the differences w(q)-w(q-1) (15) and
-# lambda (1), and writes the convective and dissipative face fluxes (15 + 15):
-# 64 doubles.
+# The roofline kernel is the face pass (k_face_jst) on a stage with
+# dissipation (stage 1), one thread per cell of [2..ie]^3.  Compulsory bytes
+# per cell: it reads the per-cell fluxes F (15), sensors (3), the differences
+# w(q)-w(q-1) (15) and lambda (1), and writes the convective and dissipative
+# face fluxes (15 + 15): 64 doubles.
 FACE_DOUBLES_DISSIP = 64
 # The Roe + viscous face pass (MUSCL states from w and p, viscous stresses
 # from the cell-centred u, v, w, T) on such a stage reads w (5), p (1) and
@@ -146,7 +146,8 @@ def kernel_roofline(case, kind, stage_ms, peak, pkind, fp64_peak):
         alg = m["alg"] * n
         ach = alg / (t * 1e-3) / 1e9 if t > 0 else 0.0
         fp = m["fp64"] * n / (t * 1e-3) if t > 0 else 0.0
-        name = {"prep": "k_prep (contracted form)", "face": "k_face_diss", "combine": "k_combine (contracted form)"}
+        name = {"prep": "k_prep (contracted form)", "face": "k_face_split (contracted form)",
+                "combine": "k_combine (contracted form)"}
         roof = {"bound": "hbm", "kernel": name[kind] + ", average launch of an update", "achieved": ach,
                 "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": m["dram"] * n,
                 "algorithmic_bytes_per_launch": alg, "launch_ms": t, "peak_kind": pkind,
