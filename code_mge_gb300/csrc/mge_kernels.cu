@@ -2141,8 +2141,9 @@ __device__ __forceinline__ void body_update(const DevBlock<T>& b, const PhysPara
 // sums variable v over the cloud (lane 5 the pressure) in the cloud's order with
 // its eight loads in flight together, and lanes 0-2 divide the normal's
 // components.  One thread a record walked the cloud 48 loads in a row, 20-34 us
-// by events; this takes 10 by itself and nothing beside the face ghosts.  Every
-// lane of a warp calls it.
+// by events; this takes 10 by itself and nothing beside the face ghosts.  All
+// eight entries are loaded: those past the cloud, and all of an empty one, hold
+// the record's own cell (mge_add_block).  Every lane of a warp calls it.
 template <typename T>
 __device__ __forceinline__ void cutcell_lanes(const DevBlock<T>& b, const PhysParams& P, unsigned* err, int t) {
   const int lane = t & 7, v = lane < 5 ? lane : 0;
@@ -2153,7 +2154,7 @@ __device__ __forceinline__ void cutcell_lanes(const DevBlock<T>& b, const PhysPa
   const long long N = b.N;
   const int ncl = b.rec_i[8 * m + 5];
   auto from = [&](T x, int l) { return __shfl_sync(0xffffffffu, x, l, 8); };
-  const int* ijk = b.rec_cloud + (8 * m + (lane < ncl ? lane : 0)) * 3;
+  const int* ijk = b.rec_cloud + (8 * m + lane) * 3;
   const int cl = (int)cidx(b.Pi, b.Pj, ijk[0], ijk[1], ijk[2]);
   const T cf = (T)b.rec_coef[8 * m + lane];
   const T* src = lane == 5 ? b.p : b.w + v * N;

@@ -932,9 +932,11 @@ int mge_add_block(mge_ctx* c, const mge_block_desc* d, int level, int serial) {
     if (t.ccid[ax] - 2 < 0 || t.ccid[ax] + 2 > lim[ax]) return fail(c, MGE_EBADCFG, "add_block: record too close to edge");
     for (int q = 0; q < MGE_MAX_CLOUD; q++) {
       t.coef[q] = d->coef[MGE_MAX_CLOUD * m + q];
+      // an entry past the cloud (all of an empty one) may hold anything: it
+      // becomes the cut cell, so that every entry is a cell of the block
       for (int e = 0; e < 3; e++) {
-        t.ijk[q][e] = d->ijkdex[(MGE_MAX_CLOUD * m + q) * 3 + e];
-        if (q < t.npoint && (t.ijk[q][e] < 0 || t.ijk[q][e] > lim[e]))
+        t.ijk[q][e] = q < t.npoint ? d->ijkdex[(MGE_MAX_CLOUD * m + q) * 3 + e] : t.ccid[e];
+        if (t.ijk[q][e] < 0 || t.ijk[q][e] > lim[e])
           return fail(c, MGE_EBADCFG, "add_block: cloud cell outside the block");
       }
     }

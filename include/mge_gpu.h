@@ -118,7 +118,7 @@ typedef struct mge_block_desc {
   const int32_t* faceid;          /* [nmir] 1..6: solid at -i,-j,-k (1,2,3) or +i,+j,+k (4,5,6) */
   const int32_t* zz;              /* [nmir] axis 1..3 */
   const int32_t* npoint;          /* [nmir] cloud size (<= MGE_MAX_CLOUD) */
-  const int32_t* ijkdex;          /* [nmir][MGE_MAX_CLOUD][3] cloud cells */
+  const int32_t* ijkdex;          /* [nmir][MGE_MAX_CLOUD][3] cloud cells; entries past npoint are not read */
   const double*  coef;            /* [nmir][MGE_MAX_CLOUD] cloud weights */
   const double*  nvec;            /* [nmir][3] wall normal (need not be unit) */
   const double*  qb;              /* [nmir][3] wall velocity; NULL = fixed wall */
