@@ -114,7 +114,10 @@ struct mge_ctx {
   std::string err;
   unsigned* d_err = nullptr;
   unsigned* h_err = nullptr;  // pinned
-  double* h_rt = nullptr;     // pinned readback of residuals
+  // pinned readback of residuals: those of a cycle, which mge_cycle_async leaves
+  // here for mge_cycle_poll, then one word for mge_euler in between
+  static constexpr int kCycleRt = 64;
+  double* h_rt = nullptr;
   double* scratch = nullptr;
   size_t bytes = 0;
   PhysParams P;
@@ -813,7 +816,7 @@ int mge_init(const mge_params* prm, int device, mge_ctx** out) {
   if (e == cudaSuccess) e = cudaMalloc(&c->d_err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMallocHost(&c->h_err, sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMallocHost(&c->h_rt, 64 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMallocHost(&c->h_rt, (mge_ctx::kCycleRt + 1) * sizeof(double));
   if (e != cudaSuccess) {
     delete c;
     return MGE_ECUDA;
@@ -1374,12 +1377,13 @@ static int euler_common(mge_ctx* c, int level, int serial, int itime, int ncyc, 
   const bool full = !lres && (nstage <= 0 || nstage >= c->prm.mstage);
   enqueue_euler(c, *b, mgl, mlvl, lres != 0, lfir != 0, nstage, full, false, itime < 0 ? 0 : itime);
   CK(cudaGetLastError());
-  if (full && ncyc >= 0) CK(cudaMemcpyAsync(c->h_rt, b->rt_cur, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  double* rt = c->h_rt + mge_ctx::kCycleRt;
+  if (full && ncyc >= 0) CK(cudaMemcpyAsync(rt, b->rt_cur, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   int rc = check_err(c);
   if (rc) return rc;
   if (full && ncyc >= 0) {
     if ((int)b->rtrms.size() <= ncyc) b->rtrms.resize(ncyc + 1, 0.0);
-    b->rtrms[ncyc] = c->h_rt[0];
+    b->rtrms[ncyc] = *rt;
   }
   return MGE_OK;
 }
@@ -1620,13 +1624,13 @@ static int launch_cycle_graph(mge_ctx* c, int mlvl_in) {
 // residual bookkeeping of solver.f90:160-181 after a cycle at FMG level mlvl
 static int read_cycle_residual(mge_ctx* c, int mlvl, int ncyc, double* max_res, double* ini_res) {
   auto& fin = c->lv[mlvl - 1];
-  for (size_t q = 0; q < fin.size() && q < 64; q++)
+  for (size_t q = 0; q < fin.size() && q < mge_ctx::kCycleRt; q++)
     CK(cudaMemcpyAsync(c->h_rt + q, fin[q].rt_cur, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaGetLastError());
   int rc = check_err(c);
   if (rc) return rc;
   double mr = 1000.0;
-  for (size_t q = 0; q < fin.size() && q < 64; q++) {
+  for (size_t q = 0; q < fin.size() && q < mge_ctx::kCycleRt; q++) {
     double r = c->h_rt[q];
     if ((int)fin[q].rtrms.size() <= ncyc) fin[q].rtrms.resize(ncyc + 1, 0.0);
     fin[q].rtrms[ncyc] = r;
@@ -1661,7 +1665,7 @@ int mge_cycle_async(mge_ctx* c, int mlvl) {
   int rc = launch_cycle_graph(c, mlvl);
   if (rc) return rc;
   auto& fin = c->lv[mlvl - 1];
-  for (size_t q = 0; q < fin.size() && q < 64; q++)
+  for (size_t q = 0; q < fin.size() && q < mge_ctx::kCycleRt; q++)
     CK(cudaMemcpyAsync(c->h_rt + q, fin[q].rt_cur, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   if (!c->ev_done) CK(cudaEventCreateWithFlags(&c->ev_done, cudaEventDisableTiming));
@@ -1688,7 +1692,7 @@ int mge_cycle_poll(mge_ctx* c, int ncyc, double* max_res) {
   }
   auto& fin = c->lv[mlvl - 1];
   double mr = 1000.0;
-  for (size_t q = 0; q < fin.size() && q < 64; q++) {
+  for (size_t q = 0; q < fin.size() && q < mge_ctx::kCycleRt; q++) {
     double r = c->h_rt[q];
     if (ncyc >= 0) {
       if ((int)fin[q].rtrms.size() <= ncyc) fin[q].rtrms.resize(ncyc + 1, 0.0);
