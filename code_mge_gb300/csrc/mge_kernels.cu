@@ -91,20 +91,31 @@ template <bool S, typename T> __device__ __forceinline__ T pmdiv(T a, T b, T y) 
   if constexpr (S) return smdiv(a, b, y); else return mdiv(a, b, y);
 }
 // Quotients by one divisor b: a/b and (a*w)/b, each operation rounded.  With the
-// integer pipes nothing is left on the FP64 pipe (soft::mulquot); without, one
-// reciprocal and Markstein's quotient.  The same bits as the divisions.
+// integer pipes nothing is left on the FP64 pipe (soft::mulquot_normal); without,
+// one reciprocal and Markstein's quotient.  The same bits as the divisions; a
+// divisor that is zero or infinite, an infinite dividend and a quotient that
+// overflows give NaN in both, as mdiv does (the time step stops there).
 template <bool S, typename T> struct SharedDiv {
   T b, y;
   __device__ __forceinline__ explicit SharedDiv(T d) : b(d), y(pdiv<S>(T(1), d)) {}
   __device__ __forceinline__ T quot(T a) const { return pmdiv<S>(a, b, y); }
   __device__ __forceinline__ T mulquot(T a, T w) const { return pmdiv<S>(pmul<S>(a, w), b, y); }
 };
+// out of line, for what lies outside the normal range
+static __device__ __noinline__ double mdiv_of(double a, double b) { return mdiv(a, b, 1.0 / b); }
+static __device__ __noinline__ double muldiv_of(double a, double w, double b) { return mdiv(a * w, b, 1.0 / b); }
 template <> struct SharedDiv<true, double> {
   double b;
   soft::Recip r;
   __device__ __forceinline__ explicit SharedDiv(double d) : b(d), r(soft::recip(d)) {}
-  __device__ __forceinline__ double quot(double a) const { return soft::quot(a, r, b); }
-  __device__ __forceinline__ double mulquot(double a, double w) const { return soft::mulquot(a, w, r, b); }
+  __device__ __forceinline__ double quot(double a) const {
+    double q;
+    return soft::quot_normal(a, r, q) ? q : mdiv_of(a, b);
+  }
+  __device__ __forceinline__ double mulquot(double a, double w) const {
+    double q;
+    return soft::mulquot_normal(a, w, r, q) ? q : muldiv_of(a, w, b);
+  }
 };
 // cell (or face) t of a box of nx by ny by any number of cells, counted from
 // (i0, i0, i0).  A block's scratch alone holds 64 fields, so its cells number

@@ -283,21 +283,20 @@ MGE_SF_HD bool quot_bits(uint64_t m, int32_t ea, uint32_t sign, const Recip& R, 
   return R.e != 0u && (uint32_t)(e - 1) < 2045u;
 }
 
-// a / b, R = recip(b)
-MGE_SF_HD double quot(double a, const Recip& R, double b) {
+// a / b, R = recip(b); false where an operand or the quotient is not a normal number
+MGE_SF_HD bool quot_normal(double a, const Recip& R, double& out) {
   const uint64_t A = bits(a);
   const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu;
-  uint64_t out;
-  if (!quot_bits((A & kFrac) | kOne, (int32_t)ea, (uint32_t)(A >> 32) & 0x80000000u, R, out) || ea - 1u >= 2046u)
-    return native_div(a, b);
-  return from_bits(out);
+  uint64_t q;
+  const bool ok = quot_bits((A & kFrac) | kOne, (int32_t)ea, (uint32_t)(A >> 32) & 0x80000000u, R, q);
+  out = from_bits(q);
+  return ok && ea - 1u < 2046u;
 }
 
-MGE_SF_NOINLINE double native_muldiv(double a, double b, double d) { return native_div(native_mul(a, b), d); }
-
 // (a * b) / d, each operation rounded, R = recip(d): mul() up to its packing,
-// then the quotient of the rounded significand
-MGE_SF_HD double mulquot(double a, double b, const Recip& R, double d) {
+// then the quotient of the rounded significand; false where an operand, the
+// product or the quotient is not a normal number
+MGE_SF_HD bool mulquot_normal(double a, double b, const Recip& R, double& out) {
   const uint64_t A = bits(a), B = bits(b);
   const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu, eb = (uint32_t)(B >> 52) & 0x7ffu;
   const int32_t e0 = (int32_t)(ea + eb) - 1023;
@@ -314,10 +313,22 @@ MGE_SF_HD double mulquot(double a, double b, const Recip& R, double d) {
   m += (rest >> 63) & ((uint64_t)((rest << 1) != 0) | (m & 1u));
   const uint32_t carry = (uint32_t)(m >> 53);
   m >>= carry;
-  uint64_t out;
-  const bool ok = quot_bits(m, e0 + (int32_t)(top + carry), (uint32_t)((A ^ B) >> 32) & 0x80000000u, R, out);
-  if (!ok || ea - 1u >= 2046u || eb - 1u >= 2046u || (uint32_t)(e0 - 1) >= 2044u) return native_muldiv(a, b, d);
-  return from_bits(out);
+  uint64_t q;
+  const bool ok = quot_bits(m, e0 + (int32_t)(top + carry), (uint32_t)((A ^ B) >> 32) & 0x80000000u, R, q);
+  out = from_bits(q);
+  return ok && ea - 1u < 2046u && eb - 1u < 2046u && (uint32_t)(e0 - 1) < 2044u;
+}
+
+MGE_SF_NOINLINE double native_muldiv(double a, double b, double d) { return native_div(native_mul(a, b), d); }
+
+// the same for all inputs, as IEEE division rounds
+MGE_SF_HD double quot(double a, const Recip& R, double b) {
+  double q;
+  return quot_normal(a, R, q) ? q : native_div(a, b);
+}
+MGE_SF_HD double mulquot(double a, double b, const Recip& R, double d) {
+  double q;
+  return mulquot_normal(a, b, R, q) ? q : native_muldiv(a, b, d);
 }
 
 }  // namespace soft
