@@ -101,6 +101,7 @@ struct PhysParams {
   int vt;                   // global time step
   int distype;              // MGE_DIS_* (0 central, 1 Roe first order, 2 Roe MUSCL)
   int irs_kind;             // 0 psmoo_old (what euler calls), 1 psmoo + progon3
+  int last_smoothed;        // psmoo_old runs in an update's last stage
   int gamma14;              // gamma is 1.4: the far field's powers take the short forms of fast_pow.cuh
   double pow_dg, pow_dm;    // gamma - 7/5 and 1/(gamma-1) - 5/2 (the double exponents' offsets)
   int unsteady;             // execmode 1: dual time stepping
@@ -249,7 +250,7 @@ template <typename T> long long bc_items(const DevBlock<T>& b, int part);
 // a level of so many cells runs so
 template <typename T> long long split_items(const DevBlock<T>& b, int e);
 void split_passes(const PhysParams& P, bool fast, long long cells, bool* prep, bool* face);
-template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* partial,
+template <typename T> void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, double* partial,
                                         int npartial, double* out, cudaStream_t s, unsigned* err = nullptr);
 template <typename T> void launch_depvars_all(const DevBlock<T>& b, const PhysParams& P, cudaStream_t s);
 template <typename T> void launch_copy_ws(const DevBlock<T>& b, cudaStream_t s);

@@ -2634,8 +2634,11 @@ int rtrms_partials(long long ncells) {
 }
 #endif
 
+// An infinite value counts as NaN where the last stage was smoothed: the sweeps turn
+// it into NaN except where their short quotient (irs_quick) leaves an infinity, and
+// the stop on the residual does not depend on the form of the sweep.
 template <typename T>
-__device__ void body_rtrms_partial(const DevBlock<T>& b, double cfl, int vt, double* partial, int npart, int part) {
+__device__ void body_rtrms_partial(const DevBlock<T>& b, const PhysParams& P, double* partial, int npart, int part) {
   __shared__ double sh[RT_THREADS];
   const long long tot = (long long)b.nx * b.ny * b.nz;
   const long long per = (tot + npart - 1) / npart;
@@ -2645,9 +2648,13 @@ __device__ void body_rtrms_partial(const DevBlock<T>& b, double cfl, int vt, dou
     int i, j, k;
     cell_of(t, b.nx, b.ny, 2, i, j, k);
     long long c = cidx(b.Pi, b.Pj, i, j, k);
-    double de = smul(cfl, (double)(vt ? *b.dtim : b.vdtim[c]));
+    double de = smul(P.cfl, (double)(P.vt ? *b.dtim : b.vdtim[c]));
     double rt = 0.0;
-    if (b.blank[c] != 0) rt = sdiv((double)b.dw[c], de);
+    if (b.blank[c] != 0) {
+      const double d = (double)b.dw[c];
+      rt = sdiv(d, de);
+      if (P.last_smoothed && ((unsigned)__double2hiint(d) & 0x7ff00000u) == 0x7ff00000u) rt = d * 0.0;
+    }
     acc = acc + smul(rt, rt);
   }
   sh[threadIdx.x] = acc;
@@ -2661,8 +2668,8 @@ __device__ void body_rtrms_partial(const DevBlock<T>& b, double cfl, int vt, dou
 }
 
 template <typename T>
-__global__ void k_rtrms_partial(DevBlock<T> b, double cfl, int vt, double* partial, int npart) {
-  body_rtrms_partial(b, cfl, vt, partial, npart, blockIdx.x);
+__global__ void k_rtrms_partial(DevBlock<T> b, PhysParams P, double* partial, int npart) {
+  body_rtrms_partial(b, P, partial, npart, blockIdx.x);
 }
 
 // The partial sums in a fixed order by one warp: lane l adds the partials
@@ -3466,7 +3473,7 @@ __global__ void __launch_bounds__(256, 1) k_euler_coop(DevBlock<T> b, PhysParams
   }
   if (E.rt) {
     for (int part = blockIdx.x; part < E.npart; part += gridDim.x)
-      body_rtrms_partial(b, P.cfl, P.vt, E.rt_partial, E.npart, part);
+      body_rtrms_partial(b, P, E.rt_partial, E.npart, part);
     g.sync();
     if (blockIdx.x == 0 && threadIdx.x < 32) body_rtrms_final(E.rt_partial, E.npart, (double)ncell, E.rt_out, E.err);
   }
@@ -3655,7 +3662,7 @@ template <typename T> struct FRtrmsPartial {
   __device__ void operator()(const MultiArgs<T>& M, int q, long long t, const DevBlock<T>& b,
                              const PhysParams& P) const {
     const int part = (int)(t / 256);
-    if (part < M.npart[q]) body_rtrms_partial(b, P.cfl, P.vt, M.rt_partial[q], M.npart[q], part);
+    if (part < M.npart[q]) body_rtrms_partial(b, P, M.rt_partial[q], M.npart[q], part);
   }
 };
 template <typename T> struct FRtrmsFinal {
@@ -4050,9 +4057,9 @@ void split_passes(const PhysParams& P, bool fast, long long cells, bool* prep, b
 #endif
 
 template <typename T>
-void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, int vt, double* partial, int npartial, double* out,
+void launch_rtrms(const DevBlock<T>& b, const PhysParams& P, double* partial, int npartial, double* out,
                   cudaStream_t s, unsigned* err) {
-  k_rtrms_partial<T><<<npartial, RT_THREADS, 0, s>>>(b, P.cfl, vt, partial, npartial);
+  k_rtrms_partial<T><<<npartial, RT_THREADS, 0, s>>>(b, P, partial, npartial);
   k_rtrms_final<<<1, 32, 0, s>>>(partial, npartial, (double)b.nx * b.ny * b.nz, out, err);
 }
 
@@ -4616,7 +4623,7 @@ void multi_movfin_level(const MultiLevel& L, const MultiPair& pair, bool fmg, cu
   template void launch_bcond<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t, bool, unsigned*);          \
   template long long bc_items<T>(const DevBlock<T>&, int);                                                      \
   template long long split_items<T>(const DevBlock<T>&, int);                                                   \
-  template void launch_rtrms<T>(const DevBlock<T>&, const PhysParams&, int, double*, int, double*, cudaStream_t, \
+  template void launch_rtrms<T>(const DevBlock<T>&, const PhysParams&, double*, int, double*, cudaStream_t, \
                                 unsigned*);                                                                    \
   template void launch_depvars_all<T>(const DevBlock<T>&, const PhysParams&, cudaStream_t);                     \
   template void launch_copy_ws<T>(const DevBlock<T>&, cudaStream_t);                                            \

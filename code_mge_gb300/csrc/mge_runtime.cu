@@ -303,7 +303,7 @@ void enqueue_euler(mge_ctx* c, Block& b, int mgl, int mlvl, bool lres, bool lfir
       if (!b.cut_beside_bcond) launch_cutcell<T>(D, c->P, c->d_err, c->stream);
       launch_bcond<T>(D, c->P, c->stream, faces_only, b.cut_beside_bcond ? c->d_err : nullptr);
     }
-    if (want_rt) launch_rtrms<T>(D, c->P, P.vt, b.rt_partial, b.npart, b.rt_cur, c->stream, c->d_err);
+    if (want_rt) launch_rtrms<T>(D, c->P, b.rt_partial, b.npart, b.rt_cur, c->stream, c->d_err);
   });
 }
 
@@ -467,6 +467,7 @@ void build_phys(mge_ctx* c) {
   Q.vt = P.vt;
   Q.distype = P.distype;
   Q.irs_kind = P.irs_variant;
+  Q.last_smoothed = P.irs_variant == 0 && P.smoo > 0.0 && P.mstage % 2 != 0;
   Q.unsteady = P.execmode == 1;
   Q.gamma14 = P.gamma == 1.4;
   Q.pow_dg = std::fma(P.gamma, 5.0, -7.0) / 5.0;    // exact 5*gamma - 7, then /5
@@ -1840,7 +1841,7 @@ int mge_kernel_times(mge_ctx* c, int level, int reps, double* ms_out, int nout) 
       rc = timed(10, [&] {
         with_dev(b, [&](auto& D) {
           using T = typename std::remove_reference_t<decltype(D)>::value_type;
-          launch_rtrms<T>(D, c->P, P.vt, b.rt_partial, b.npart, b.rt_cur, c->stream);
+          launch_rtrms<T>(D, c->P, b.rt_partial, b.npart, b.rt_cur, c->stream);
         });
       });
   }
