@@ -14,8 +14,9 @@
 //   k_rec_*    per cut-cell record: the efluxb/dfluxb face replacements
 //   k_combine  per cell: dw, fw, forcing, blanking, time-step scaling and,
 //              without smoothing, the update + depvars (euler.f90:127-399)
-//   k_irs_*    implicit residual smoothing lines (psmoo.f90:171-237), the
-//              k-line fused with the update
+//   k_irs_*    implicit residual smoothing lines (psmoo.f90:171-237)
+//   k_update   the state after smoothing and depvars (euler.f90:375-399)
+//   k_bcond    boundary conditions and the records' solid states
 //
 // Arithmetic follows the reference expression by expression.  The plain path
 // is compiled with --fmad=false (no contraction); divisions by a quantity
@@ -145,9 +146,11 @@ __device__ __forceinline__ double irs_e1(const IrsTables& t, int q, double) { re
 __device__ __forceinline__ float irs_e1(const IrsTables& t, int q, float) { return t.e1f[q]; }
 __device__ __forceinline__ double irs_e1r(const IrsTables& t, int q, double) { return t.e1r[q]; }
 __device__ __forceinline__ float irs_e1r(const IrsTables& t, int q, float) { return t.e1rf[q]; }
-// x / e1[q] as fma(x, e1r, x*e1l), with e1r + e1l = 1/e1 to twice the precision
-// (the host has checked that this rounds as the division for every x,
-// IrsTables::quick): one dependent operation fewer than Markstein's quotient
+// x / e1[q] as fma(x, e1r, x*e1l), with e1r + e1l = 1/e1 to twice the precision: one
+// dependent operation fewer than Markstein's quotient.  The host has checked that
+// it rounds as the division for every finite x whose products and quotient are
+// normal numbers (IrsTables::quick).  An infinite x gives infinity or NaN by the
+// sign of e1l, where mdiv gives NaN; the residual norm counts both as NaN.
 template <bool SC> __device__ __forceinline__ double irs_quick(double x, double e1r, double e1l) {
   return fma(x, e1r, SC ? smul(x, e1l) : x * e1l);
 }
@@ -312,9 +315,6 @@ __global__ void k_timestep(DevBlock<T> b, PhysParams P, unsigned* err) {
   block_min_dtim(mine, b.dtim, gridDim.x);  // global dtim (timestep.f90:112), kept even when vt = 0
 }
 
-template <typename T> __global__ void k_set_scalar(T* p, double v) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *p = (T)v;
-}
 // --------------------------------------------------------------- stage: per-cell pass
 // Box [1..ie]x[1..je]x[1..ke]: every cell whose flux or sensor a face needs.
 template <bool S, typename T>
@@ -448,7 +448,6 @@ __device__ __forceinline__ void body_prep_dir(const DevBlock<T>& b, const PhysPa
     pm = b.p[c - st], pp = b.p[c + st];
   }
   const T y = pdiv<S>(T(1), w[0]), Hc = w[4] + p;
-  if (P.matrix) b.H[c] = Hc;
   const T s = (T)b.s[D];
   const T f0 = pmul<S>(w[1 + D], s);
   T f[5];

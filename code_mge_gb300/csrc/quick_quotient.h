@@ -8,7 +8,7 @@
 namespace mge {
 
 // The low part yl of 1/y, yh = RN(1/y), for which fma(x, yh, RN(x*yl)) is the
-// correctly rounded x/y for every x (products and quotient in the normal
+// correctly rounded x/y for every finite x (products and quotient in the normal
 // range): N. Brisebarre, J.-M. Muller, S. K. Raina, Accelerating correctly
 // rounded floating-point division when the divisor is known in advance, IEEE
 // Trans. Computers 53(8), 2004.  The value before the last rounding is within
