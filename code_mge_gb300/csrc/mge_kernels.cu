@@ -3758,7 +3758,11 @@ inline int tpb_for(long long n) {
 // FP64 blocks of up to this many cells run plain FP64 operations instead of
 // the integer-pipe forms (pmul).  Measured, plain against integer: a W-cycle's
 // 24^3 update 269 against 281 us, a 64x64x2 one 402 against 421; a 48^3 level's
-// cycle 1.18 against 1.09 ms, a 192^3 one 50 against 40.
+// cycle 1.18 against 1.09 ms, a 192^3 one 50 against 40.  The line is the central
+// scheme's.  An update of the upwind schemes crosses over earlier, first-order Roe
+// and MUSCL with NS, ms: 64x64x2 0.345 against 0.403 and 0.511 against 0.574, 24^3 0.320
+// against 0.355 and 0.501 against 0.527, 128x64x2 0.457 against 0.465 and 0.714 against
+// 0.660, 128x128x2 0.616 against 0.585 and 0.993 against 0.828.
 constexpr long long kPlainCells = 32768;
 template <typename T> bool on_int_pipes(const DevBlock<T>& b) {
   return (long long)b.nx * b.ny * b.nz > kPlainCells;
